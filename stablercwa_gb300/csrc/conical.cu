@@ -991,8 +991,7 @@ void conical_schur_modes(Batch& c, const std::vector<SchurJob>& jobs, std::vecto
         zc* Tc = mem.get<zc>((size_t)per);
         int* infoc = mem.zeros<int>(total);
         zc* wsc = mem.get<zc>((size_t)(eig_workspace_bytes(n, total) / sizeof(zc)) + 1);
-        const int group = eig_group ? eig_group : eig_default_group(n, total);
-        launch_eig(st, n, total, Hc, nn, wc, Zc, infoc, nullptr, wsc, 2.220446049250313e-16, 100, group, nullptr, 0, Tc);
+        launch_eig(st, n, total, Hc, nn, wc, Zc, infoc, nullptr, wsc, 2.220446049250313e-16, 100, eig_group, nullptr, 0, Tc);
         LAUNCH(scatter_flagged_kernel, nblocks(per), kTpb, st, total, nn, dptrs + J, dmap, Zc);
         LAUNCH(scatter_flagged_kernel, nblocks(per), kTpb, st, total, nn, dptrs + 2 * J, dmap, Tc);
         LAUNCH(scatter_flagged_info_kernel, nblocks(total), kTpb, st, total, dinfos, dmap, infoc);

@@ -28,9 +28,28 @@ int eig_default_group(int n, int batch) {
     return batch * 32LL * 4 >= lanes_wanted ? 32 : 128;
 }
 
+namespace {
+// the FP64 kernels with `group` lanes or threads per matrix
+void launch_eig_fp64(cudaStream_t st, int n, int batch, const zc* a, long long a_stride, zc* w, zc* v, int* info, int* sweeps,
+                     zc* ws, double eps, int max_iter, int group, const int* skip, int skip_value, zc* t_out);
+}  // namespace
+
 void launch_eig(cudaStream_t st, int n, int batch, const zc* a, long long a_stride, zc* w, zc* v, int* info, int* sweeps,
                 zc* ws, double eps, int max_iter, int group, const int* skip, int skip_value, zc* t_out) {
     if (batch <= 0 || n <= 0) return;
+    // The fixed-point solver wherever it can hold the order and the call asks for nothing of the FP64 iteration's
+    // own (a forced form, its sweep counts, other tolerances or caps); what it leaves unfinished goes on to the
+    // FP64 kernels. The autotuner's table chooses among the FP64 forms, for the calls that take those.
+    if (group == 0 && !skip && !sweeps && eps == DBL_EPSILON && max_iter >= 30 && eig_fixed_possible(n)) {
+        TimedLaunch timed(TK_EIG, st);
+        int* done = nullptr;
+        RCWA_CUDA(cudaMallocAsync(&done, (size_t)batch * sizeof(int), st));
+        launch_eig_fixed(st, n, batch, a, a_stride, w, v, info, ws, done, eps, t_out);
+        launch_eig_fp64(st, n, batch, a, a_stride, w, v, info, sweeps, ws, eps, max_iter, eig_default_group(n, batch), done, 1,
+                        t_out);
+        RCWA_CUDA(cudaFreeAsync(done, st));
+        return;
+    }
     if (group == 0 && !skip && !t_out) {
         if (autotune_wanted(0, n, batch)) autotune_eig(st, 0, n, batch, a, a_stride, nullptr);
         group = tuned_eig_form(0, n, batch);
@@ -42,6 +61,12 @@ void launch_eig(cudaStream_t st, int n, int batch, const zc* a, long long a_stri
     }
     if (group <= 0) group = eig_default_group(n, batch);
     TimedLaunch timed(TK_EIG, st);
+    launch_eig_fp64(st, n, batch, a, a_stride, w, v, info, sweeps, ws, eps, max_iter, group, skip, skip_value, t_out);
+}
+
+namespace {
+void launch_eig_fp64(cudaStream_t st, int n, int batch, const zc* a, long long a_stride, zc* w, zc* v, int* info, int* sweeps,
+                     zc* ws, double eps, int max_iter, int group, const int* skip, int skip_value, zc* t_out) {
     if (group > 32) {
         switch (group) {
             case 64: eig_block_kernel<64><<<(unsigned)batch, 64, 0, st>>>(n, batch, a, a_stride, w, v, info, sweeps, ws, eps, max_iter, skip, skip_value, t_out); break;
@@ -66,6 +91,7 @@ void launch_eig(cudaStream_t st, int n, int batch, const zc* a, long long a_stri
     ++launch_count();
     RCWA_CUDA(cudaGetLastError());
 }
+}  // namespace
 
 // QL rotations applied by the Hermitian eigensolver since the last read (the work of its sweeps, 12 n flops
 // each, for the benchmark's roofline)

@@ -1,0 +1,91 @@
+// eig_fixed.cu -- launcher of the fixed-point general eigensolver (kernels in eig_fixed.cuh).
+#include <algorithm>
+#include <cstdlib>
+
+#include "eig_fixed.cuh"
+#include "engine.h"
+
+namespace rcwa_gb300 {
+namespace {
+
+// largest order: 32 rows of Z (16 bytes an entry) and the back substitution's slots in 227 KB of shared memory
+constexpr int kFixMaxOrder = 440;
+constexpr int kFixMinOrder = 24;
+// Matrices per pass: the logs (about 96 n^2 bytes each) of half the batch, so that they stay within what the
+// callers' estimates leave beside the eigensolver's workspace, but of three matrices an SM at least and of 4 GB
+// at most.
+constexpr int kFixPassMin = 456;
+constexpr long long kFixLogBytes = 4LL << 30;
+
+bool fix_enabled() {
+    static const bool on = [] {
+        const char* e = std::getenv("RCWA_GB300_EIG_FIXED");
+        return !(e && e[0] == '0');
+    }();
+    return on;
+}
+
+// warps of fix_schur_kernel's CTA: a lane per row or column of the matrix up to order 352 (11 warps' tiles are
+// what shared memory holds), at least four so that three warps trail the one that forms the rotations
+int fix_warps(int n) { return std::min(11, std::max(4, (n + 31) / 32)); }
+
+}  // namespace
+
+bool eig_fixed_possible(int n) { return fix_enabled() && n >= kFixMinOrder && n <= kFixMaxOrder; }
+
+long long eig_fixed_bytes(int n) {
+    if (!eig_fixed_possible(n)) return 0;
+    return 2 * fix_log_capacity(n) * (long long)sizeof(int4) + fix_table_capacity(n) * (long long)sizeof(int4);
+}
+
+void launch_eig_fixed(cudaStream_t st, int n, int batch, const zc* a, long long a_stride, zc* w, zc* v, int* info, zc* ws,
+                      int* done, double eps, zc* t_out) {
+    const long long nn = (long long)n * n, wst = (3 * nn + 4LL * n + 8);  // eig_workspace_elems
+    const int warps = fix_warps(n);
+    const size_t schur_smem = fix_schur_smem(n, warps), row_smem = (size_t)n * 32 * sizeof(lz),
+                 back_smem = (size_t)(n + 4) * 32 * sizeof(zc);
+    ensure_smem_optin(reinterpret_cast<const void*>(fix_schur_kernel), (int)schur_smem);
+    if (row_smem > 46 * 1024) ensure_smem_optin(reinterpret_cast<const void*>(fix_apply_kernel), (int)row_smem);
+    if (back_smem > 48 * 1024) ensure_smem_optin(reinterpret_cast<const void*>(fix_backsub_kernel), (int)back_smem);
+    const int chunk = (int)std::max(1LL, std::min<long long>(std::min(batch, std::max(kFixPassMin, (batch + 1) / 2)),
+                                                             kFixLogBytes / eig_fixed_bytes(n)));
+    int4 *log = nullptr, *table = nullptr;
+    int *head = nullptr, *status = nullptr;
+    unsigned long long* tn = nullptr;
+    RCWA_CUDA(cudaMallocAsync(&log, (size_t)chunk * 2 * fix_log_capacity(n) * sizeof(int4), st));
+    RCWA_CUDA(cudaMallocAsync(&table, (size_t)chunk * fix_table_capacity(n) * sizeof(int4), st));
+    RCWA_CUDA(cudaMallocAsync(&head, (size_t)chunk * 2 * sizeof(int), st));
+    RCWA_CUDA(cudaMallocAsync(&status, (size_t)chunk * sizeof(int), st));
+    RCWA_CUDA(cudaMallocAsync(&tn, (size_t)chunk * sizeof(unsigned long long), st));
+    for (int b0 = 0; b0 < batch; b0 += chunk) {
+        const int cb = std::min(chunk, batch - b0);
+        const zc* ac = a + (long long)b0 * a_stride;
+        zc *wc = w + (long long)b0 * n, *vc = v + (long long)b0 * nn, *wsc = ws + (long long)b0 * wst;
+        zc *z1 = wsc + nn, *z2 = wsc + 2 * nn;  // Z; X
+        lz* h = reinterpret_cast<lz*>(wsc);
+        fix_schur_kernel<<<(unsigned)cb, 32 * warps, schur_smem, st>>>(n, cb, ac, a_stride, wc, h, wst, log, table, head, status,
+                                                                       done + b0, info + b0);
+        RCWA_CUDA(cudaGetLastError());
+        fix_apply_kernel<<<dim3((unsigned)cb, (unsigned)((n + 31) / 32)), 32, row_smem, st>>>(n, cb, z1, wst, log, table, head, status);
+        RCWA_CUDA(cudaGetLastError());
+        zc* t = t_out ? t_out + (long long)b0 * nn : vc;
+        RCWA_CUDA(cudaMemsetAsync(tn, 0, (size_t)cb * sizeof(unsigned long long), st));
+        fix_triangle_kernel<<<(unsigned)((nn * cb + 255) / 256), 256, 0, st>>>(n, cb, h, wst, t, nn, wc, head, status, tn);
+        RCWA_CUDA(cudaGetLastError());
+        launch_count() += 3;
+        if (t_out) {  // the Schur form: T and Z
+            RCWA_CUDA(cudaMemcpy2DAsync(vc, nn * sizeof(zc), z1, wst * sizeof(zc), nn * sizeof(zc), cb, cudaMemcpyDeviceToDevice, st));
+            continue;
+        }
+        fix_backsub_kernel<<<dim3((unsigned)cb, (unsigned)((n + 31) / 32)), kFixBackThreads, back_smem, st>>>(
+            n, cb, t, nn, wc, tn, z2, wst, status, eps);
+        RCWA_CUDA(cudaGetLastError());
+        launch_zgemm_untimed(st, n, n, n, cb, z1, n, wst, z2, n, wst, nullptr, 0, vc, n, nn, 1.0, 0.0, status, 1);
+        fix_unit_columns_kernel<<<(unsigned)(((long long)cb * n * 32 + 127) / 128), 128, 0, st>>>(n, cb, vc, nn, status);
+        RCWA_CUDA(cudaGetLastError());
+        launch_count() += 2;
+    }
+    for (void* p : {(void*)log, (void*)table, (void*)head, (void*)status, (void*)tn}) RCWA_CUDA(cudaFreeAsync(p, st));
+}
+
+}  // namespace rcwa_gb300

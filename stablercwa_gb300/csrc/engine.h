@@ -103,6 +103,13 @@ bool eig_cluster_possible(int n, int batch);
 void preload_eig_cluster_kernel();
 void launch_eig_cluster(cudaStream_t st, int n, int batch, const zc* a, long long a_stride, zc* w, zc* v, int* info,
                         int* sweeps, zc* ws, double eps, int max_iter, const int* skip, int skip_value, zc* t_out);
+// The general eigensolver with its unitary transformations in fixed point (eig_fixed.cu), for orders it can hold
+// (eig_fixed_possible): done[b] = 1 for every matrix it finished (info[b] = 0), 0 for one it leaves to the FP64
+// kernels. ws as launch_eig's; it allocates eig_fixed_bytes(n) a matrix besides (up to 4 GB at a time).
+bool eig_fixed_possible(int n);
+long long eig_fixed_bytes(int n);
+void launch_eig_fixed(cudaStream_t st, int n, int batch, const zc* a, long long a_stride, zc* w, zc* v, int* info, zc* ws,
+                      int* done, double eps, zc* t_out);
 // The same product on the tensor cores (gemm_tc.cu: Ozaki-split bf16 tcgen05 products, FP64-accurate);
 // launch_zgemm takes it for products of order >= 32 unless RCWA_GB300_GEMM=fp64. The triangular hint
 // does not apply (the full product is formed; zero entries contribute exact zeros).

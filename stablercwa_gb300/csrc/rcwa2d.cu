@@ -501,7 +501,8 @@ void solve2d_host(cudaStream_t st, const rcwa_stack2d& stack, const rcwa_point2d
     }
 
     // ---- chunk size from a per-point estimate of the device working set
-    double per_point = 16.0 * (double)nn * (5.0 * P + 3.0 * (L + 1) + 8.0) + 64.0 * N * (L + 8);
+    double per_point = 16.0 * (double)nn * (5.0 * P + 3.0 * (L + 1) + 8.0) + 64.0 * N * (L + 8) +
+                       (double)P * (double)eig_fixed_bytes(n);
     if (nz > 0)  // retained W, V and reflections, amplitudes, the field output and one depth group's buffers
         per_point += 16.0 * ((double)nn * (2.0 * P + L) + 4.0 * n * L + 12.0 * (double)N * nz);
     const int B_max = (int)std::max(1.0, std::min((double)valid.size(), (double)chunk_bytes / per_point));
