@@ -19,15 +19,14 @@
 // times k) and one final rounding: FP64-level accuracy with S = 7.
 //
 // Kernels. The split kernels write the digit planes in HBM as bf16 rows with K contiguous (K-major for
-// both operands). The product kernel gives each CTA one 128 x 128 tile of C^ of one matrix: one warp
-// issues TMA loads (128-byte swizzle, boxes of 128 rows x 64 K) into a 4-stage shared-memory ring; one
-// thread issues tcgen05.mma (M = 128, N = 128, K = 16, bf16 in, FP32 out) into one of two 128-column
-// tensor-memory accumulators; eight warps read each finished group out of tensor memory (tcgen05.ld) and
-// add it, as an integer at its diagonal's weight, into one int64 per element while the next group
-// accumulates in the other buffer, then convert once, apply 2^(ea + eb), pair the real and imaginary rows
-// and write C. Every mbarrier wait is bounded: on
-// expiry the kernel records an error, drains its own copies and products, frees its tensor memory and
-// returns without writing C.
+// both operands), the second half of a complex K starting at Kp / 2. The product kernel gives each CTA one
+// 128 x 128 tile of C^ of one matrix: one warp issues TMA loads (128-byte swizzle, boxes of 128 rows x 64 K, two
+// of each operand a stage) into a 3-stage shared-memory ring; one thread issues tcgen05.mma (M = 128, N = 128,
+// K = 16, bf16 in, FP32 out) into one of two 128-column tensor-memory accumulators; eight warps read each finished
+// group out of tensor memory (tcgen05.ld) and add it, as an integer at its diagonal's weight, into one int64 per
+// element while the next group accumulates in the other buffer, then convert once, apply 2^(ea + eb), pair the
+// real and imaginary rows and write C. Every mbarrier wait is bounded: on expiry the kernel records an error,
+// drains its own copies and products, frees its tensor memory and returns without writing C.
 #include <cuda.h>
 #include <cuda_runtime.h>
 
@@ -43,9 +42,14 @@
 namespace rcwa_gb300 {
 namespace {
 
-constexpr int kTileM = 128, kTileN = 128, kTileK = 64;  // K per stage: 64 bf16 = one 128-byte swizzle row
-constexpr int kStages = 4;
-constexpr int kStageBytes = (kTileM + kTileN) * kTileK * 2;  // 32 KB
+// A stage holds 128 K of both operands (64 bf16 = one 128-byte swizzle row a box): with the 64 K of an earlier form
+// the issuing thread's wait, eight descriptors and commit took 560 cycles a stage against the 256 of its four
+// MMAs; eight MMAs a stage and descriptors that are additions keep the tensor pipe ahead.
+constexpr int kTileM = 128, kTileN = 128, kTileK = 64;
+constexpr int kStageBoxes = 2;
+constexpr int kStages = 3;
+constexpr int kBoxBytes = kTileM * kTileK * 2;               // 16 KB
+constexpr int kStageBytes = 2 * kStageBoxes * kBoxBytes;      // A boxes, then B boxes: 64 KB
 constexpr int kTmemCols = 256;                                // two accumulators of 128 columns
 constexpr int kThreads = 320;                                 // producer, MMA, 8 epilogue warps
 constexpr int kMaxGroups = 160;
@@ -133,16 +137,19 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
-    uint32_t r[16];
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
+    uint32_t r[32];
     asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,"
+        "%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]),
+          "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]),
+          "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
         : "r"(taddr));
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-    for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
+    for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
 }
 
 // ---------------------------------------------------------------- digit split
@@ -197,36 +204,6 @@ __device__ __forceinline__ long long fixed62(double x, int e) {
     return (b >> 63) ? -(long long)m : (long long)m;
 }
 
-// x 2^e2 as the nearest double (ties to even), for |x| < 2^63, from integer operations only: the FP64 pipe
-// of this GPU runs 1/32 of the FP32 rate, so the epilogue's conversions would otherwise dominate the tile.
-// False when the result is not a normal double (the caller converts in FP64 then).
-__device__ __forceinline__ bool i64_ldexp_bits(long long x, int e2, unsigned long long& bits) {
-    if (x == 0) {
-        bits = 0;
-        return true;
-    }
-    const unsigned long long sign = x < 0 ? 0x8000000000000000ull : 0ull;
-    const unsigned long long u = x < 0 ? 0ull - (unsigned long long)x : (unsigned long long)x;
-    const int msb = 63 - __clzll((long long)u);
-    int ex = msb + e2;
-    unsigned long long mant;
-    if (msb > 52) {
-        const int r = msb - 52;
-        const unsigned long long rem = u & ((1ull << r) - 1ull), half = 1ull << (r - 1);
-        mant = u >> r;
-        if (rem > half || (rem == half && (mant & 1ull))) ++mant;
-        if (mant >> 53) {
-            mant >>= 1;
-            ++ex;
-        }
-    } else {
-        mant = u << (52 - msb);
-    }
-    if (ex < -1022 || ex > 1023) return false;
-    bits = sign | ((unsigned long long)(ex + 1023) << 52) | (mant & 0xFFFFFFFFFFFFFull);
-    return true;
-}
-
 // c as an integer count of 2^e2 units (nearest, ties to even), for adding C0 into the accumulator; false when
 // c is subnormal, not finite, or at least 2^61 units (the caller adds in FP64 then)
 __device__ __forceinline__ bool double_to_units(double c, int e2, long long& t) {
@@ -253,66 +230,81 @@ __device__ __forceinline__ bool double_to_units(double c, int e2, long long& t) 
     return true;
 }
 
-// bf16 bit pattern of a small integer (exact for |d| <= 256), from integer operations
-__device__ __forceinline__ uint16_t bf16_int(long long d) {
-    if (d == 0) return 0;
-    const unsigned sign = d < 0 ? 0x8000u : 0u;
-    const unsigned a = (unsigned)(d < 0 ? -d : d);
-    const int p = 31 - __clz((int)a);  // a = 1.f 2^p
-    return (uint16_t)(sign | ((unsigned)(p + 127) << 7) | ((a << (7 - p)) & 0x7Fu));
+// The digits of x 2^-e (|x 2^-e| < 1), all at once. With Y = |x| 2^(62 - e) rounded to 62 fractional bits, the bytes
+// of W = 2 (Y + sum_{s >= 1} 2^(62 - 8 s) + half a unit of the last digit) are the digits of |x| 2^-e: the top byte
+// is d_0 in [0, 128] itself and each lower one d_s + 128 with d_s in [-128, 127] (the added 2^(62 - 8 s) are the
+// offsets 128; carries have moved up already). Digit s has weight 2^(-7 - 8 s); x's sign goes onto every digit. An
+// eighth digit is byte 0. A non-finite x (whose row or column then carries kNonFinite) gives zero digits.
+struct DigitWord {
+    unsigned hi, lo, sign;  // sign 0x8000 for a negative x
+};
+// Y of a zero or subnormal x, or one in a row or column with a non-finite entry (out of line: rare)
+__device__ __noinline__ unsigned long long digit_y_slow(double x, int e) {
+    return mag_bits(x) >= kMagInf || e == kNonFinite ? 0ull : (unsigned long long)fixed62(fabs(x), e);
 }
-
-// The S digits of x 2^-e (|x 2^-e| < 1), integer arithmetic: Y = x 2^(62 - e) is the value to 62 fractional
-// bits (an int64 below 2^62, so adding the rounding half never overflows); digit s (from 0) is Y rounded at
-// bit 55 - 8 s and taken out of Y before the next, so each lies in [-128, 128] and carries weight
-// 2^(-7 - 8 s); an eighth digit is the remainder itself, in units of 2^-63. A non-finite x (whose row or
-// column then carries kNonFinite) gives zero digits.
-__device__ __forceinline__ void split_digits(double x, int e, int S, uint16_t* dg) {
-    if (mag_bits(x) >= kMagInf || e == kNonFinite) {
-        for (int s = 0; s < S; ++s) dg[s] = 0;
-        return;
-    }
-    long long Y = fixed62(x, e);
-#pragma unroll 1
-    for (int s = 0; s < S; ++s) {
-        const int sh = 55 - 8 * s;
-        long long d;
-        if (sh > 0) {
-            d = (Y + (1LL << (sh - 1))) >> sh;
-            Y -= d * (1LL << sh);
-        } else {
-            d = Y * (1LL << -sh);
-            Y = 0;
-        }
-        dg[s] = bf16_int(d);
-    }
+__device__ __forceinline__ unsigned long long digit_offsets(int S) {
+    unsigned long long c = 1ull << (54 - 8 * (min(S, 7) - 1));
+    for (int s = 1; s < min(S, 7); ++s) c += 1ull << (62 - 8 * s);
+    return c;
 }
-
-__device__ __forceinline__ void store_digits(double x, int e, int S, uint16_t* out, long long plane_stride) {
-    if (mag_bits(x) >= kMagInf || e == kNonFinite) {
-        for (int s = 0; s < S; ++s) out[s * plane_stride] = 0;
-        return;
-    }
-    long long Y = fixed62(x, e);
-#pragma unroll 1
-    for (int s = 0; s < S; ++s) {
-        const int sh = 55 - 8 * s;
-        long long d;
-        if (sh > 0) {
-            d = (Y + (1LL << (sh - 1))) >> sh;
-            Y -= d * (1LL << sh);
-        } else {
-            d = Y * (1LL << -sh);
-            Y = 0;
-        }
-        out[s * plane_stride] = bf16_int(d);
-    }
+__device__ __forceinline__ DigitWord digit_word(double x, int e, unsigned long long offsets) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+    const int be = (int)((b >> 52) & 0x7FF);
+    const unsigned long long mant = ((b & 0xFFFFFFFFFFFFFull) | (1ull << 52)) << 9;  // |x| = mant 2^(be - 1084)
+    const int r = min(1022 + e - be, 63);                                           // |x| < 2^e keeps it >= 0
+    unsigned long long Y = (mant + ((1ull << (r & 63)) >> 1)) >> (r & 63);
+    if (be == 0 || be == 0x7FF || e == kNonFinite) Y = (b << 1) == 0 ? 0ull : digit_y_slow(x, e);
+    const unsigned long long W = (Y + offsets) << 1;
+    return DigitWord{(unsigned)(W >> 32), (unsigned)W, (unsigned)(b >> 48) & 0x8000u};
+}
+// digit s of two values as a pair of bf16 (the first in the low half), signs not yet applied: 128 + (byte & 127)
+// and 128, 256 or 0 are exact in bf16, and so is their difference
+template <int s>
+__device__ __forceinline__ unsigned digit_pair(const DigitWord& a, const DigitWord& b) {
+    constexpr unsigned byte = s < 4 ? 3 - s : 7 - s;
+    const unsigned u = __byte_perm(s < 4 ? a.hi : a.lo, s < 4 ? b.hi : b.lo, byte | (byte + 4) << 8);
+    const unsigned x = (u & 0x007f007fu) | 0x43004300u;
+    const unsigned c = s == 0 ? 0x43004300u - (u & 0x00800080u) * 0x86u : (u & 0x00800080u) ^ 0x43804380u;
+    unsigned d;
+    asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(x), "r"(c));
+    return d;
+}
+// the S digits of four consecutive values of a row to the planes at out (8-byte aligned), and with a second place
+// the same with the signs flipped there if `flip`
+template <int s>
+__device__ __forceinline__ void store_digit(const DigitWord* w, unsigned sg01, unsigned sg23, uint16_t* out, uint16_t* out2,
+                                            unsigned flip, long long plane) {
+    const unsigned d01 = digit_pair<s>(w[0], w[1]) ^ sg01, d23 = digit_pair<s>(w[2], w[3]) ^ sg23;
+    *reinterpret_cast<uint2*>(out + s * plane) = make_uint2(d01, d23);
+    if (out2) *reinterpret_cast<uint2*>(out2 + s * plane) = make_uint2(d01 ^ flip, d23 ^ flip);
+}
+__device__ __forceinline__ void store_digits4(const double* x, int e, int S, unsigned long long offsets, uint16_t* out, uint16_t* out2,
+                                              unsigned flip, long long plane) {
+    DigitWord w[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) w[j] = digit_word(x[j], e, offsets);
+    // a value that is zero (or in a non-finite row) has all digits zero whatever its sign: -0 times a finite digit is
+    // a zero, which the sums ignore
+    const unsigned sg01 = w[0].sign | w[1].sign << 16, sg23 = w[2].sign | w[3].sign << 16;
+    store_digit<0>(w, sg01, sg23, out, out2, flip, plane);
+    if (S > 1) store_digit<1>(w, sg01, sg23, out, out2, flip, plane);
+    if (S > 2) store_digit<2>(w, sg01, sg23, out, out2, flip, plane);
+    if (S > 3) store_digit<3>(w, sg01, sg23, out, out2, flip, plane);
+    if (S > 4) store_digit<4>(w, sg01, sg23, out, out2, flip, plane);
+    if (S > 5) store_digit<5>(w, sg01, sg23, out, out2, flip, plane);
+    if (S > 6) store_digit<6>(w, sg01, sg23, out, out2, flip, plane);
+    if (S > 7) store_digit<7>(w, sg01, sg23, out, out2, flip, plane);
 }
 
 // A (m x k, column-major, lda) of matrix blockIdx.y -> S planes of A^ (2m rows x Kp, K contiguous) and
 // ea[i]; one CTA per 32 rows of A. Complex B (real_b = 0): rows 2i, 2i+1 = [Re A(i,:), -Im A(i,:)] and
-// [Im A(i,:), Re A(i,:)] over K = 2k; real B (real_b = 1): rows [Re A(i,:)] and [Im A(i,:)] over K = k.
-// A is read through a shared-memory tile (coalesced along the rows) and written row by row.
+// [Im A(i,:), Re A(i,:)], the second part from Kp / 2 on, zeros after k of each; real B (real_b = 1): rows
+// [Re A(i,:)] and [Im A(i,:)] over K = k.
+// A is read through a shared-memory tile (coalesced along the rows); a thread then splits four consecutive entries
+// of a row and stores them as eight bytes a plane. Bound by integer instructions and the planes' writes: 0.29 us a
+// matrix of order 121 (304 of them; 867 KB of planes each, 3.0 TB/s), against 0.90 us of the digit-by-digit form with
+// two-byte stores before it.
+constexpr int kSplitTile = 32;
 __global__ void __launch_bounds__(256) tc_split_a_kernel(int m, int k, int Kp, int S, int real_b, const zc* __restrict__ A,
                                                          int lda, long long a_stride, uint16_t* __restrict__ out,
                                                          int* __restrict__ ea) {
@@ -321,13 +313,15 @@ __global__ void __launch_bounds__(256) tc_split_a_kernel(int m, int k, int Kp, i
     const zc* As = A + b * a_stride;
     __shared__ unsigned long long smax[8][32];
     __shared__ int sexp[32];
-    __shared__ zc tile[32][33];
+    __shared__ zc tile[32][kSplitTile + 1];
     unsigned long long mx = 0;
-    if (i0 + il < m)
+    if (i0 + il < m) {
+#pragma unroll 4
         for (int kk = w; kk < k; kk += 8) {
             const zc v = As[(long long)kk * lda + i0 + il];
             mx = max(mx, max(mag_bits(v.re), mag_bits(v.im)));
         }
+    }
     smax[w][il] = mx;
     __syncthreads();
     if (w == 0) {
@@ -335,106 +329,151 @@ __global__ void __launch_bounds__(256) tc_split_a_kernel(int m, int k, int Kp, i
         sexp[il] = scale_exponent(mx);
         if (i0 + il < m) ea[b * m + i0 + il] = sexp[il];
     }
-    __syncthreads();
-    const long long rows = 2LL * m, plane = rows * Kp;
+    const long long plane = 2LL * m * Kp;
     uint16_t* o = out + b * S * plane;
-    const int kin = real_b ? k : 2 * k;  // K of the product before padding
-    for (int kc = 0; kc < k; kc += 32) {
-        for (int q = w; q < 32; q += 8) {
-            const int kk = kc + q, i = i0 + il;
-            tile[il][q] = (kk < k && i < m) ? As[(long long)kk * lda + i] : zc{0.0, 0.0};
+    const int half = real_b ? Kp : Kp / 2;
+    const unsigned long long offsets = digit_offsets(S);
+    const int r = t >> 3, i = i0 + r, q4 = 4 * (t & 7);  // the row and the four columns this thread splits
+    for (int kc = 0; kc < half; kc += kSplitTile) {
+        __syncthreads();
+        for (int q = w; q < kSplitTile; q += 8) {
+            const int kk = kc + q;
+            tile[il][q] = (kk < k && i0 + il < m) ? As[(long long)kk * lda + i0 + il] : zc{0.0, 0.0};
         }
         __syncthreads();
-        // each value is split once: Re A(i, kk) goes to row 2i at kk and row 2i+1 at k + kk, Im A(i, kk) to row
-        // 2i+1 at kk and, negated digit by digit (the negated digits sum exactly to -Im A), to row 2i at k + kk
-        for (int idx = t; idx < 64 * 32; idx += 256) {
-            const int vi = idx >> 5, c = idx & 31, kk = kc + c;
-            const int il2 = vi >> 1, im_part = vi & 1, i = i0 + il2;
-            if (i >= m || kk >= k) continue;
-            const zc v = tile[il2][c];
-            uint16_t dg[kMaxSlices];
-            split_digits(im_part ? v.im : v.re, sexp[il2], S, dg);
-            uint16_t* first = o + (2LL * i + im_part) * Kp + kk;
-            for (int s2 = 0; s2 < S; ++s2) first[s2 * plane] = dg[s2];
-            if (!real_b) {
-                uint16_t* second = o + (2LL * i + (1 - im_part)) * Kp + k + kk;
-                for (int s2 = 0; s2 < S; ++s2)
-                    second[s2 * plane] = im_part && dg[s2] ? (uint16_t)(dg[s2] ^ 0x8000u) : dg[s2];
-            }
-        }
-        __syncthreads();
-    }
-    for (int idx = t; idx < 64 * (Kp - kin); idx += 256) {  // zero padding of K
-        const int rr = idx / (Kp - kin), kk = kin + idx - rr * (Kp - kin);
-        const int i = i0 + (rr >> 1), part = rr & 1;
         if (i >= m) continue;
-        uint16_t* cell = o + (2LL * i + part) * Kp + kk;
-        for (int s2 = 0; s2 < S; ++s2) cell[s2 * plane] = 0;
+        const int e = sexp[r];
+        double re[4], im[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const zc v = tile[r][q4 + j];
+            re[j] = v.re;
+            im[j] = v.im;
+        }
+        uint16_t* row0 = o + 2LL * i * Kp + kc + q4;
+        uint16_t* row1 = row0 + Kp;
+        store_digits4(re, e, S, offsets, row0, real_b ? nullptr : row1 + half, 0u, plane);
+        store_digits4(im, e, S, offsets, row1, real_b ? nullptr : row0 + half, 0x80008000u, plane);
     }
 }
 
-// B (k x n, column-major, ldb) -> S planes of B^t (n rows x Kp) and eb[j]; one warp per column. Complex B:
-// [Re B(:, j); Im B(:, j)]; real B (Br, double): B(:, j).
+// B (k x n, column-major, ldb) -> S planes of B^t (n rows x Kp) and eb[j]; G = 8, 16 or 32 lanes per column (so that
+// a k of 32, the factorisations' updates, keeps all lanes busy), four consecutive entries a lane. Complex B:
+// [Re B(:, j); Im B(:, j)], the imaginary part from Kp / 2 on; real B (Br, double): B(:, j); zeros after k.
+// Order 121 (304 matrices): 0.15 us a matrix against 0.42 us with two-byte stores.
+template <int G>
 __global__ void __launch_bounds__(128) tc_split_b_kernel(int n, int k, int Kp, int S, int batch, const zc* __restrict__ B,
                                                          const double* __restrict__ Br, int ldb, long long b_stride,
                                                          uint16_t* __restrict__ out, int* __restrict__ eb) {
-    const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / G;
     if (gw >= (long long)batch * n) return;
+    const unsigned mask = group_mask<G>();
     const long long b = gw / n;
-    const int j = (int)(gw - b * n), lane = threadIdx.x & 31;
+    const int j = (int)(gw - b * n), lane = threadIdx.x & (G - 1);
+    const zc* col = Br ? nullptr : B + b * b_stride + (long long)j * ldb;
+    const double* rcol = Br ? Br + b * b_stride + (long long)j * ldb : nullptr;
     unsigned long long mx = 0;
     if (Br) {
-        const double* col = Br + b * b_stride + (long long)j * ldb;
-        for (int kk = lane; kk < k; kk += 32) mx = max(mx, mag_bits(col[kk]));
+#pragma unroll 4
+        for (int kk = lane; kk < k; kk += G) mx = max(mx, mag_bits(rcol[kk]));
     } else {
-        const zc* col = B + b * b_stride + (long long)j * ldb;
-        for (int kk = lane; kk < k; kk += 32) mx = max(mx, max(mag_bits(col[kk].re), mag_bits(col[kk].im)));
+#pragma unroll 4
+        for (int kk = lane; kk < k; kk += G) mx = max(mx, max(mag_bits(col[kk].re), mag_bits(col[kk].im)));
     }
-    for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    for (int o = G / 2; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(mask, mx, o, G));
     const int e = scale_exponent(mx);
     if (lane == 0) eb[b * n + j] = e;
     const long long plane = (long long)n * Kp;
     uint16_t* o = out + b * S * plane + (long long)j * Kp;
-    for (int kk = lane; kk < Kp; kk += 32) {
-        double x;
-        if (Br) {
-            x = kk < k ? Br[b * b_stride + (long long)j * ldb + kk] : 0.0;
-        } else {
-            const zc* col = B + b * b_stride + (long long)j * ldb;
-            x = kk < k ? col[kk].re : (kk < 2 * k ? col[kk - k].im : 0.0);
+    const unsigned long long offsets = digit_offsets(S);
+    const int half = Br ? Kp : Kp / 2;
+    for (int kk = 4 * lane; kk < half; kk += 4 * G) {
+        double re[4], im[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const bool in = kk + u < k;
+            if (Br) {
+                re[u] = in ? rcol[kk + u] : 0.0;
+            } else {
+                const zc v = in ? col[kk + u] : zc{0.0, 0.0};
+                re[u] = v.re;
+                im[u] = v.im;
+            }
         }
-        store_digits(x, e, S, o + kk, plane);
+        store_digits4(re, e, S, offsets, o + kk, nullptr, 0u, plane);
+        if (!Br) store_digits4(im, e, S, offsets, o + kk + half, nullptr, 0u, plane);
     }
+}
+void split_b(cudaStream_t st, int n, int k, int Kp, int S, int batch, const zc* B, const double* Br, int ldb, long long b_stride,
+             uint16_t* out, int* eb) {
+    const int half = Br ? Kp : Kp / 2, g = half <= 32 ? 8 : half <= 64 ? 16 : 32;
+    const unsigned blocks = (unsigned)(((long long)batch * n * g + 127) / 128);
+    if (g == 8) tc_split_b_kernel<8><<<blocks, 128, 0, st>>>(n, k, Kp, S, batch, B, Br, ldb, b_stride, out, eb);
+    else if (g == 16) tc_split_b_kernel<16><<<blocks, 128, 0, st>>>(n, k, Kp, S, batch, B, Br, ldb, b_stride, out, eb);
+    else tc_split_b_kernel<32><<<blocks, 128, 0, st>>>(n, k, Kp, S, batch, B, Br, ldb, b_stride, out, eb);
+    ++launch_count();
 }
 
 // ---------------------------------------------------------------- the product
 
-// One element of C from its int64 accumulator ac (units of 2^(e - 14 - s0)), e = ea + eb: s_ab = +-1 and
-// s_c in {0, 1} (unit_scales) without FP64 arithmetic (C0's part joins as an integer count of the same unit,
-// one rounding to double by integer operations), anything else in FP64; NaN for a non-finite row or column.
-__device__ __forceinline__ double finish_element(long long ac, int e, int s0, bool neg, bool unit_scales, const double* C0d,
-                                                 long long off2, double s_ab, double s_c) {
+// One element of C from its int64 accumulator ac (units of 2^(e - 14 - s0)), e = ea + eb; NaN for a non-finite row or
+// column. With s_ab = +-1 and s_c in {0, 1} (unit_scales, every product of the solves) C0's part joins as an integer
+// count of the same unit and the sum is rounded once, to nearest even, by integer operations. (The conversion
+// instruction runs on the FP64 pipe: with two warps a scheduler 322 cycles an element against 260.) What is not
+// a normal double then, or has other scales, is rare and out of line: inlined, its instructions were issued
+// (predicated off) for every element.
+__device__ __noinline__ double finish_slow(long long ac, int e, int s0, double c0, double s_ab, double s_c) {
     if (e >= kNonFinite / 2) return __longlong_as_double(0x7FF8000000000000LL);
+    return fma(s_c, c0, s_ab * ldexp((double)ac, e - 14 - s0));
+}
+template <bool HasC0>
+__device__ __forceinline__ double finish_element(long long ac, int e, int s0, long long neg, bool unit_scales, double c0, double s_ab,
+                                                 double s_c) {
     const int e2 = e - 14 - s0;
-    long long a = neg ? -ac : ac;
+    long long a = (ac ^ neg) - neg;  // neg: 0 or -1
     bool fast = unit_scales;
-    if (fast && C0d) {
+    if (HasC0) {
         long long t;
-        fast = double_to_units(C0d[off2], e2, t);
+        fast = double_to_units(c0, e2, t) && fast;
         a += t;
     }
-    unsigned long long bits;
-    if (fast && i64_ldexp_bits(a, e2, bits)) return __longlong_as_double((long long)bits);
-    double out = s_ab * ldexp((double)ac, e2);
-    if (C0d) out = fma(s_c, C0d[off2], out);
-    return out;
+    const unsigned long long u = (unsigned long long)(a < 0 ? -a : a);  // below 2^63
+    const int lz = __clzll((long long)u);
+    const unsigned long long w = u << ((lz - 1) & 63);  // the leading one at bit 62
+    const unsigned long long q = (w + 0x1FF + ((unsigned)(w >> 10) & 1u)) >> 10;  // 53 bits, or 2^53: the sum below carries it
+    const int ex = 1085 - lz + e2;  // biased exponent - 1
+    fast = fast && (a == 0 ? e < kNonFinite / 2 : (unsigned)ex < 2045u);
+    if (!fast) return finish_slow(ac, e, s0, HasC0 ? c0 : 0.0, s_ab, HasC0 ? s_c : 0.0);
+    const int hi = (int)(q >> 32) + (ex << 20) + (a < 0 ? (int)0x80000000 : 0);
+    return __hiloint2double(a == 0 ? 0 : hi, a == 0 ? 0 : (int)q);
 }
 
 struct SharedState {
     uint64_t full[kStages], empty[kStages], tfull[2], tempty[2], drain;
     uint32_t tmem_base;
     int abort_flag;
+    int eb[kTileN];  // the columns' scale exponents
 };
+
+// acc += x 2^sh (rounded for sh < 0) for 32 group sums x = v (integers below 2^24; x 2^sh stays below 2^62)
+__device__ __forceinline__ void add_group(long long* acc, const float* v, int sh) {
+    if (sh >= 32) {
+        const int k = sh - 32;
+#pragma unroll
+        for (int j = 0; j < 32; ++j) acc[j] += (long long)((unsigned long long)(unsigned)(__float2int_rn(v[j]) << k) << 32);
+    } else if (sh >= 0) {
+        const int dbl = sh == 31, f = 1 << (sh - dbl);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+            const int x = __float2int_rn(v[j]) << dbl;
+            asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(acc[j]) : "r"(x), "r"(f));
+        }
+    } else {
+        const int half = 1 << (-sh - 1);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) acc[j] += (long long)((__float2int_rn(v[j]) + half) >> -sh);
+    }
+}
 
 __global__ void __launch_bounds__(kThreads, 1)
     tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ Plan plan,
@@ -470,6 +509,10 @@ __global__ void __launch_bounds__(kThreads, 1)
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
         tc_fence_before();
     }
+    if (warp >= 2 && warp < 6) {
+        const int j = threadIdx.x - 64;
+        ss->eb[j] = n0 + j < n ? eb[(long long)(b_bcast ? 0 : batch0 + lb) * n + n0 + j] : 0;
+    }
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = ss->tmem_base;
@@ -479,35 +522,42 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (warp == 0) {
         // ---- TMA producer
         if (lane == 0) {
-            int it = 0;
-            int issued[kStages];
-            for (int s = 0; s < kStages; ++s) issued[s] = -1;
+            int st = 0, ph = 1, issued = 0;
             bool ok = true;
             for (int gi = 0; gi < plan.n_groups && ok; ++gi) {
                 const unsigned g = plan.g[gi];
-                const int d = g_d(g);
-                for (int p = 0; p < g_ni(g) && ok; ++p) {
-                    const int i = g_i0(g) + p, j = d - i;
-                    for (int kb = g_kb0(g); kb < g_kb0(g) + g_nkb(g); ++kb, ++it) {
-                        const int st = it % kStages, ph = (it / kStages) & 1;
-                        if (!mbar_wait(&ss->empty[st], ph ^ 1, abort_flag, err)) {
+                const int d = g_d(g), i0 = g_i0(g), ni = g_ni(g), kb0 = g_kb0(g), kb1 = kb0 + g_nkb(g);
+                for (int p = 0; p < ni && ok; ++p) {
+                    const int pa = za * S + i0 + p - 1, pb = zb * S + d - i0 - p - 1;
+                    for (int kb = kb0; kb < kb1; kb += kStageBoxes) {
+                        if (!mbar_wait(&ss->empty[st], ph, abort_flag, err)) {
                             ok = false;
                             break;
                         }
                         unsigned char* sa = smem + st * kStageBytes;
-                        mbar_expect_tx(&ss->full[st], kStageBytes);
-                        tma_load_3d(sa, &map_a, kb * kTileK, m0, za * S + i - 1, &ss->full[st]);
-                        tma_load_3d(sa + kTileM * kTileK * 2, &map_b, kb * kTileK, n0, zb * S + j - 1, &ss->full[st]);
-                        issued[st] = it;
+                        uint64_t* full = &ss->full[st];
+                        const bool two = kb + 1 < kb1;
+                        mbar_expect_tx(full, two ? kStageBytes : kStageBytes / 2);
+                        tma_load_3d(sa, &map_a, kb * kTileK, m0, pa, full);
+                        tma_load_3d(sa + kStageBoxes * kBoxBytes, &map_b, kb * kTileK, n0, pb, full);
+                        if (two) {
+                            tma_load_3d(sa + kBoxBytes, &map_a, (kb + 1) * kTileK, m0, pa, full);
+                            tma_load_3d(sa + (kStageBoxes + 1) * kBoxBytes, &map_b, (kb + 1) * kTileK, n0, pb, full);
+                        }
+                        ++issued;
+                        if (++st == kStages) {
+                            st = 0;
+                            ph ^= 1;
+                        }
                     }
                 }
             }
             if (!ok) {
                 // drain: wait (bounded) for the copies this thread started into each stage
                 for (int s = 0; s < kStages; ++s) {
-                    if (issued[s] < 0) continue;
-                    const int ph = (issued[s] / kStages) & 1;
-                    for (unsigned r = 0; r < kWaitLimit && !mbar_try_wait(&ss->full[s], ph); ++r) {
+                    const int uses = (issued + kStages - 1 - s) / kStages;
+                    if (uses == 0) continue;
+                    for (unsigned r = 0; r < kWaitLimit && !mbar_try_wait(&ss->full[s], (uses - 1) & 1); ++r) {
                     }
                 }
             }
@@ -515,12 +565,13 @@ __global__ void __launch_bounds__(kThreads, 1)
     } else if (warp == 1) {
         // ---- MMA issuer
         if (lane == 0) {
-            int it = 0;
+            const uint64_t base = smem_desc_sw128(smem_u32(smem));
+            int st = 0, ph = 0;
             bool ok = true;
             bool any = false;
             for (int gi = 0; gi < plan.n_groups && ok; ++gi) {
                 const unsigned g = plan.g[gi];
-                const int buf = gi & 1;
+                const int buf = gi & 1, ni = g_ni(g), nkb = g_nkb(g);
                 if (!mbar_wait(&ss->tempty[buf], ((gi >> 1) & 1) ^ 1, abort_flag, err)) {
                     ok = false;
                     break;
@@ -528,23 +579,31 @@ __global__ void __launch_bounds__(kThreads, 1)
                 tc_fence_after();
                 const uint32_t d_tmem = tmem + buf * kTileN;
                 uint32_t acc = 0;
-                for (int p = 0; p < g_ni(g) && ok; ++p) {
-                    for (int kb = 0; kb < g_nkb(g); ++kb, ++it) {
-                        const int st = it % kStages, ph = (it / kStages) & 1;
+                for (int p = 0; p < ni && ok; ++p) {
+                    for (int kb = 0; kb < nkb; kb += kStageBoxes) {
                         if (!mbar_wait(&ss->full[st], ph, abort_flag, err)) {
                             ok = false;
                             break;
                         }
                         tc_fence_after();
-                        const uint32_t a_addr = smem_u32(smem + st * kStageBytes);
-                        const uint32_t b_addr = a_addr + kTileM * kTileK * 2;
+                        // descriptors count 16-byte units: 32 bytes of K further is + 2, a box is + 1024
+                        const uint64_t da = base + (uint64_t)st * (kStageBytes >> 4), db = da + (kStageBoxes * kBoxBytes >> 4);
 #pragma unroll
                         for (int kk = 0; kk < kTileK / 16; ++kk) {
-                            mma_bf16(d_tmem, smem_desc_sw128(a_addr + kk * 32), smem_desc_sw128(b_addr + kk * 32), acc);
+                            mma_bf16(d_tmem, da + 2 * kk, db + 2 * kk, acc);
                             acc = 1;
+                        }
+                        if (kb + 1 < nkb) {
+#pragma unroll
+                            for (int kk = 0; kk < kTileK / 16; ++kk)
+                                mma_bf16(d_tmem, da + (kBoxBytes >> 4) + 2 * kk, db + (kBoxBytes >> 4) + 2 * kk, 1);
                         }
                         any = true;
                         mma_commit(&ss->empty[st]);  // the stage is free once these products have read it
+                        if (++st == kStages) {
+                            st = 0;
+                            ph ^= 1;
+                        }
                     }
                 }
                 if (ok) mma_commit(&ss->tfull[buf]);
@@ -575,22 +634,16 @@ __global__ void __launch_bounds__(kThreads, 1)
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             tc_fence_after();
-            const int d = g_d(plan.g[gi]);
-            const int sh = plan.s0 - 8 * (d - 2);
+            const int sh = plan.s0 - 8 * (g_d(plan.g[gi]) - 2);
             const uint32_t base = tmem + ((uint32_t)(q * 32) << 16) + buf * kTileN + h * 64;
-            const int lsh = sh >= 0 ? sh : 0, rsh = sh >= 0 ? 0 : -sh;  // one of them is zero
-            const long long half = rsh ? (1LL << (rsh - 1)) : 0LL;
-#pragma unroll
-            for (int c16 = 0; c16 < 4; ++c16) {
-                float v[16];
-                tmem_ld16(base + c16 * 16, v);
-#pragma unroll
-                for (int j = 0; j < 16; ++j)
-                    acc[c16 * 16 + j] += (((long long)__float2int_rn(v[j]) << lsh) + half) >> rsh;
-            }
+            float v[32];
+            tmem_ld32(base, v);
+            add_group(acc, v, sh);
+            tmem_ld32(base + 32, v);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&ss->tempty[buf]);
+            add_group(acc + 32, v, sh);
         }
         if (ok && !*abort_flag) {
             // Each lane writes its own row's part of C: row r of C^ is the real (r even) or imaginary part of
@@ -601,28 +654,36 @@ __global__ void __launch_bounds__(kThreads, 1)
             const int r = m0 + q * 32 + lane;  // row of A^
             const int i = r >> 1, part = r & 1;
             const int er = (i < m) ? ea[(long long)(a_bcast ? 0 : batch0 + lb) * m + i] : 0;
-            const int* ebs = eb + (long long)(b_bcast ? 0 : batch0 + lb) * n;
             double* Cd = reinterpret_cast<double*>(C + (long long)(batch0 + lb) * c_stride);
             const double* C0d = C0 && s_c != 0.0 ? reinterpret_cast<const double*>(C0 + (long long)(batch0 + lb) * c0_stride)
                                                  : nullptr;
             const bool unit_scales = (s_ab == 1.0 || s_ab == -1.0) && (C0d == nullptr || s_c == 1.0);
-            const bool neg = s_ab < 0.0;
             // The accumulators go to shared memory first (the stage ring is idle once the last group has
             // landed; column-major by thread, so a warp's accesses are conflict-free), which keeps the
             // conversion loop below out of the registers that hold them.
             long long* sacc = reinterpret_cast<long long*>(smem);
-            const int et = threadIdx.x - 64;
+            const int et = threadIdx.x - 64, cols = min(64, n - n0 - h * 64);
 #pragma unroll
             for (int c = 0; c < 64; ++c) sacc[c * 256 + et] = acc[c];
             if (i < m) {
-#pragma unroll 2
-                for (int c = 0; c < 64; ++c) {
-                    const int col = n0 + h * 64 + c;
-                    if (col >= n) break;
-                    const long long ac = sacc[c * 256 + et];
-                    const int e = er + ebs[col];
-                    const long long off2 = 2 * ((long long)col * ldc + i) + part;
-                    Cd[off2] = finish_element(ac, e, plan.s0, neg, unit_scales, C0d, off2, s_ab, s_c);
+                const int* se = ss->eb + h * 64;
+                const long long step = 2LL * ldc, neg = s_ab < 0.0 ? -1 : 0;
+                long long off2 = 2 * ((long long)(n0 + h * 64) * ldc + i) + part;
+                if (C0d) {
+                    for (int c = 0; c < cols; c += 4, off2 += 4 * step) {
+                        double c0v[4];
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) c0v[u] = c + u < cols ? C0d[off2 + u * step] : 0.0;
+#pragma unroll
+                        for (int u = 0; u < 4; ++u)
+                            if (c + u < cols)
+                                Cd[off2 + u * step] = finish_element<true>(sacc[(c + u) * 256 + et], er + se[c + u], plan.s0, neg,
+                                                                           unit_scales, c0v[u], s_ab, s_c);
+                    }
+                } else {
+#pragma unroll 4
+                    for (int c = 0; c < cols; ++c, off2 += step)
+                        Cd[off2] = finish_element<false>(sacc[c * 256 + et], er + se[c], plan.s0, neg, unit_scales, 0.0, s_ab, s_c);
                 }
             }
         }
@@ -632,246 +693,6 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (warp == 1) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
-    }
-}
-
-// ---------------------------------------------------------------- the slice-resident product
-//
-// The same product with each operand tile loaded once per K block instead of once per digit pair: a CTA
-// computes a 128 x 64 tile of C^; per K block of 64 the producer loads the S slices of B's 64 rows (one B
-// stage, S x 8 KB, double-buffered) and then the S slices of A's 128 rows one after another (a 4-deep
-// ring of 16 KB), and A slice s meets every B slice t with s + t <= S - 1 (0-based) while it is resident:
-// 4 MMAs (M 128, N 64, K 16) per pair into the tensor-memory accumulator of its diagonal s + t (S
-// accumulators of 64 columns). 168 KB of operand tiles feed 28 pairs per K block for S = 7, against 32 KB
-// per pair in the kernel above: about 2.7x fewer bytes per MMA. Every accumulator sums at most S pairs over
-// K chunks of 128 (S x 128 x 2^14 <= 2^24, exact in FP32); after each chunk the eight epilogue warps add
-// the S accumulators into their int64 registers at each diagonal's weight (the same units as above) while
-// the MMA warp waits for them, then the last chunk's sums are converted as above.
-constexpr int kTileNr = 64;                                   // columns of C^ per CTA
-constexpr int kBStage = kMaxSlices * kTileNr * kTileK * 2;     // one K block of every B slice: 64 KB
-constexpr int kATile = kTileM * kTileK * 2;                    // one A slice tile: 16 KB
-constexpr int kARing = 4;
-constexpr int kChunkKb = 2;                                    // K blocks per exact accumulation chunk
-constexpr uint32_t kIdescN64 = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kTileNr >> 3) << 17) |
-                               ((uint32_t)(kTileM >> 4) << 24);
-
-__device__ __forceinline__ void mma_bf16_n64(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(d_tmem),
-        "l"(adesc), "l"(bdesc), "r"(kIdescN64), "r"(accumulate)
-        : "memory");
-}
-
-struct SharedStateR {
-    uint64_t afull[kARing], aempty[kARing], bfull[2], bempty[2], tfull, tempty, drain;
-    uint32_t tmem_base;
-    int abort_flag;
-};
-
-__global__ void __launch_bounds__(kThreads, 1)
-    tc_gemm_resident_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, int S,
-                            int s0, int kblocks, int m, int n, int batch0, int a_bcast, int b_bcast,
-                            const int* __restrict__ ea, const int* __restrict__ eb, const zc* C0, long long c0_stride,
-                            zc* C, int ldc, long long c_stride, double s_ab, double s_c, const int* __restrict__ skip,
-                            int skip_value, int* __restrict__ err) {
-    const int lb = blockIdx.z;
-    if (skip && skip[batch0 + lb] == skip_value) return;
-    extern __shared__ __align__(1024) unsigned char smem_raw[];
-    unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    unsigned char* bst = smem;                    // 2 B stages
-    unsigned char* ast = smem + 2 * kBStage;      // the A ring
-    SharedStateR* ss = reinterpret_cast<SharedStateR*>(ast + kARing * kATile);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int m0 = blockIdx.y * kTileM, n0 = blockIdx.x * kTileNr;
-    const int nchunks = (kblocks + kChunkKb - 1) / kChunkKb;
-
-    if (threadIdx.x == 0) {
-        for (int r = 0; r < kARing; ++r) {
-            mbar_init(&ss->afull[r], 1);
-            mbar_init(&ss->aempty[r], 1);
-        }
-        for (int r = 0; r < 2; ++r) {
-            mbar_init(&ss->bfull[r], 1);
-            mbar_init(&ss->bempty[r], 1);
-        }
-        mbar_init(&ss->tfull, 1);
-        mbar_init(&ss->tempty, 8);
-        mbar_init(&ss->drain, 1);
-        ss->abort_flag = 0;
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&ss->tmem_base)),
-                     "r"(512)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-        tc_fence_before();
-    }
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem = ss->tmem_base;
-    volatile int* abort_flag = &ss->abort_flag;
-    const int za = a_bcast ? 0 : lb, zb = b_bcast ? 0 : lb;
-
-    if (warp == 0) {
-        // ---- TMA producer: per K block one B stage (all slices), then the A slices through the ring
-        if (lane == 0) {
-            bool ok = true;
-            int ai = 0, bi = 0;
-            int aissued[kARing], bissued[2];
-            for (int r = 0; r < kARing; ++r) aissued[r] = -1;
-            bissued[0] = bissued[1] = -1;
-            for (int kb = 0; kb < kblocks && ok; ++kb) {
-                const int b = bi & 1, bph = (bi >> 1) & 1;
-                if (!mbar_wait(&ss->bempty[b], bph ^ 1, abort_flag, err)) {
-                    ok = false;
-                    break;
-                }
-                mbar_expect_tx(&ss->bfull[b], (uint32_t)(S * kTileNr * kTileK * 2));
-                for (int t = 0; t < S; ++t)
-                    tma_load_3d(bst + b * kBStage + t * (kTileNr * kTileK * 2), &map_b, kb * kTileK, n0, zb * S + t,
-                                &ss->bfull[b]);
-                bissued[b] = bi;
-                ++bi;
-                for (int sl = 0; sl < S; ++sl, ++ai) {
-                    const int r = ai % kARing, aph = (ai / kARing) & 1;
-                    if (!mbar_wait(&ss->aempty[r], aph ^ 1, abort_flag, err)) {
-                        ok = false;
-                        break;
-                    }
-                    mbar_expect_tx(&ss->afull[r], (uint32_t)kATile);
-                    tma_load_3d(ast + r * kATile, &map_a, kb * kTileK, m0, za * S + sl, &ss->afull[r]);
-                    aissued[r] = ai;
-                }
-            }
-            if (!ok) {  // drain: wait (bounded) for the copies this thread started
-                for (int r = 0; r < kARing; ++r) {
-                    if (aissued[r] < 0) continue;
-                    const int ph = (aissued[r] / kARing) & 1;
-                    for (unsigned it = 0; it < kWaitLimit && !mbar_try_wait(&ss->afull[r], ph); ++it) {
-                    }
-                }
-                for (int r = 0; r < 2; ++r) {
-                    if (bissued[r] < 0) continue;
-                    const int ph = (bissued[r] >> 1) & 1;
-                    for (unsigned it = 0; it < kWaitLimit && !mbar_try_wait(&ss->bfull[r], ph); ++it) {
-                    }
-                }
-            }
-        }
-    } else if (warp == 1) {
-        // ---- MMA issuer
-        if (lane == 0) {
-            bool ok = true, any = false;
-            int ai = 0, bi = 0;
-            for (int c = 0; c < nchunks && ok; ++c) {
-                if (!mbar_wait(&ss->tempty, (c & 1) ^ 1, abort_flag, err)) {
-                    ok = false;
-                    break;
-                }
-                tc_fence_after();
-                const int kb0 = c * kChunkKb, kb1 = min(kblocks, kb0 + kChunkKb);
-                for (int kb = kb0; kb < kb1 && ok; ++kb) {
-                    const int b = bi & 1, bph = (bi >> 1) & 1;
-                    if (!mbar_wait(&ss->bfull[b], bph, abort_flag, err)) {
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after();
-                    const uint32_t b_base = smem_u32(bst + b * kBStage);
-                    for (int sl = 0; sl < S; ++sl, ++ai) {
-                        const int r = ai % kARing, aph = (ai / kARing) & 1;
-                        if (!mbar_wait(&ss->afull[r], aph, abort_flag, err)) {
-                            ok = false;
-                            break;
-                        }
-                        tc_fence_after();
-                        const uint32_t a_addr = smem_u32(ast + r * kATile);
-                        for (int t = 0; t + sl < S; ++t) {
-                            const uint32_t b_addr = b_base + t * (kTileNr * kTileK * 2);
-                            const uint32_t d_tmem = tmem + (uint32_t)((sl + t) * kTileNr);
-#pragma unroll
-                            for (int kk = 0; kk < kTileK / 16; ++kk) {
-                                const uint32_t acc = (kb == kb0 && sl == 0 && kk == 0) ? 0u : 1u;
-                                mma_bf16_n64(d_tmem, smem_desc_sw128(a_addr + kk * 32), smem_desc_sw128(b_addr + kk * 32),
-                                             acc);
-                            }
-                        }
-                        any = true;
-                        mma_commit(&ss->aempty[r]);  // the A tile is free once these products have read it
-                    }
-                    if (!ok) break;
-                    mma_commit(&ss->bempty[b]);
-                    ++bi;
-                }
-                if (ok) mma_commit(&ss->tfull);
-            }
-            if (!ok && any) {
-                mma_commit(&ss->drain);
-                for (unsigned it = 0; it < kWaitLimit && !mbar_try_wait(&ss->drain, 0); ++it) {
-                }
-            }
-        }
-    } else {
-        // ---- epilogue: warps 2..9; lane quarter q of tensor memory, column half h (32 of the 64 columns)
-        const int q = warp & 3, h = (warp - 2) >> 2;
-        long long acc[32];
-#pragma unroll
-        for (int cc = 0; cc < 32; ++cc) acc[cc] = 0;
-        bool ok = true;
-        for (int c = 0; c < nchunks; ++c) {
-            ok = mbar_wait(&ss->tfull, c & 1, abort_flag, err);
-            ok = __all_sync(0xffffffffu, ok);
-            if (!ok) break;
-            tc_fence_after();
-            for (int dg = 0; dg < S; ++dg) {  // diagonal dg = s + t enters at 2^(s0 - 8 dg)
-                const int sh = s0 - 8 * dg;
-                const int lsh = sh >= 0 ? sh : 0, rsh = sh >= 0 ? 0 : -sh;
-                const long long half = rsh ? (1LL << (rsh - 1)) : 0LL;
-                const uint32_t base = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(dg * kTileNr + h * 32);
-#pragma unroll
-                for (int c16 = 0; c16 < 2; ++c16) {
-                    float v[16];
-                    tmem_ld16(base + c16 * 16, v);
-#pragma unroll
-                    for (int j = 0; j < 16; ++j)
-                        acc[c16 * 16 + j] += (((long long)__float2int_rn(v[j]) << lsh) + half) >> rsh;
-                }
-            }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&ss->tempty);
-        }
-        if (ok && !*abort_flag) {
-            const int r = m0 + q * 32 + lane;  // row of A^
-            const int i = r >> 1, part = r & 1;
-            const int er = (i < m) ? ea[(long long)(a_bcast ? 0 : batch0 + lb) * m + i] : 0;
-            const int* ebs = eb + (long long)(b_bcast ? 0 : batch0 + lb) * n;
-            double* Cd = reinterpret_cast<double*>(C + (long long)(batch0 + lb) * c_stride);
-            const double* C0d = C0 && s_c != 0.0 ? reinterpret_cast<const double*>(C0 + (long long)(batch0 + lb) * c0_stride)
-                                                 : nullptr;
-            const bool unit_scales = (s_ab == 1.0 || s_ab == -1.0) && (C0d == nullptr || s_c == 1.0);
-            const bool neg = s_ab < 0.0;
-            long long* sacc = reinterpret_cast<long long*>(ast);  // the A ring is idle after the last chunk
-            const int et = threadIdx.x - 64;
-#pragma unroll
-            for (int cc = 0; cc < 32; ++cc) sacc[cc * 256 + et] = acc[cc];
-            if (i < m) {
-#pragma unroll 2
-                for (int cc = 0; cc < 32; ++cc) {
-                    const int col = n0 + h * 32 + cc;
-                    if (col >= n) break;
-                    const long long off2 = 2 * ((long long)col * ldc + i) + part;
-                    Cd[off2] = finish_element(sacc[cc * 256 + et], er + ebs[col], s0, neg, unit_scales, C0d, off2, s_ab, s_c);
-                }
-            }
-        }
-    }
-    tc_fence_before();
-    __syncthreads();
-    if (warp == 1) {
-        tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
     }
 }
 
@@ -895,12 +716,12 @@ EncodeTiled encode_fn() {
     return fn;
 }
 
-// digit planes (planes x rows x Kp bf16, K contiguous) as a 3-D tensor map with 64 x box_rows boxes
-CUtensorMap plane_map(const uint16_t* base, long long rows, int Kp, long long planes, int box_rows = kTileM) {
+// digit planes (planes x rows x Kp bf16, K contiguous) as a 3-D tensor map with 64 x 128 boxes
+CUtensorMap plane_map(const uint16_t* base, long long rows, int Kp, long long planes) {
     CUtensorMap map;
     const cuuint64_t dims[3] = {(cuuint64_t)Kp, (cuuint64_t)rows, (cuuint64_t)planes};
     const cuuint64_t strides[2] = {(cuuint64_t)Kp * 2, (cuuint64_t)rows * Kp * 2};
-    const cuuint32_t box[3] = {(cuuint32_t)kTileK, (cuuint32_t)box_rows, 1};
+    const cuuint32_t box[3] = {(cuuint32_t)kTileK, (cuuint32_t)kTileM, 1};
     const cuuint32_t estr[3] = {1, 1, 1};
     const CUresult r = encode_fn()(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<uint16_t*>(base), dims, strides,
                                    box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
@@ -937,19 +758,6 @@ Plan make_plan(int S, int kblocks) {
 int* error_flag() { return static_cast<int*>(device_word(1, sizeof(int))); }
 
 }  // namespace
-
-// the slice-resident kernel when RCWA_GB300_TC_KERNEL=resident. Not the default: it moves 2.7x fewer bytes
-// from L2 per MMA but measured slower (4096 products of order 121: 9.8 ms against 8.8 ms; tensor pipe 17 %
-// against 22 %): its tiles are half as wide, so twice the CTAs pay the per-tile setup and epilogue, and its
-// single set of accumulators makes the MMAs wait for every chunk's drain. A persistent form that overlaps
-// one tile's epilogue with the next tile's products is what it needs.
-bool tc_gemm_resident() {
-    static const bool on = [] {
-        const char* e = std::getenv("RCWA_GB300_TC_KERNEL");
-        return e && std::strcmp(e, "resident") == 0;
-    }();
-    return on;
-}
 
 int tc_gemm_slices() {
     static const int s = [] {
@@ -988,11 +796,8 @@ void tc_product(cudaStream_t st, int m, int n, int k, int batch, const zc* A, in
                 const double* Br, int ldb, long long b_stride, const zc* C0, long long c0_stride, zc* C, int ldc,
                 long long c_stride, double s_ab, double s_c, const int* skip, int skip_value) {
     if (batch <= 0 || m <= 0 || n <= 0) return;
-    const bool resident = tc_gemm_resident();
-    const int smem_bytes = resident ? 2 * kBStage + kARing * kATile + 1024 + (int)sizeof(SharedStateR) + 64
-                                    : kStages * kStageBytes + 1024 + (int)sizeof(SharedState) + 64;
-    if (resident) ensure_smem_optin(reinterpret_cast<const void*>(tc_gemm_resident_kernel), smem_bytes);
-    else ensure_smem_optin(reinterpret_cast<const void*>(tc_gemm_kernel), smem_bytes);
+    const int smem_bytes = kStages * kStageBytes + 1024 + (int)sizeof(SharedState) + 64;
+    ensure_smem_optin(reinterpret_cast<const void*>(tc_gemm_kernel), smem_bytes);
     const int real_b = Br != nullptr;
     const int S = tc_gemm_slices();
     const int kin = real_b ? k : 2 * k;
@@ -1013,14 +818,13 @@ void tc_product(cudaStream_t st, int m, int n, int k, int batch, const zc* A, in
     RCWA_CUDA(cudaMallocAsync(&dea, sizeof(int) * (size_t)m * (a_bcast ? 1 : batch), st));
     RCWA_CUDA(cudaMallocAsync(&deb, sizeof(int) * (size_t)n * (b_bcast ? 1 : batch), st));
     const CUtensorMap map_a = plane_map(pa, 2LL * m, Kp, (long long)na * S);
-    const CUtensorMap map_b = plane_map(pb, n, Kp, (long long)nb * S, resident ? kTileNr : kTileN);
+    const CUtensorMap map_b = plane_map(pb, n, Kp, (long long)nb * S);
     if (a_bcast) {
         tc_split_a_kernel<<<dim3((m + 31) / 32, 1), 256, 0, st>>>(m, k, Kp, S, real_b, A, lda, 0, pa, dea);
         ++launch_count();
     }
     if (b_bcast) {
-        tc_split_b_kernel<<<(unsigned)((n * 32LL + 127) / 128), 128, 0, st>>>(n, k, Kp, S, 1, B, Br, ldb, 0, pb, deb);
-        ++launch_count();
+        split_b(st, n, k, Kp, S, 1, B, Br, ldb, 0, pb, deb);
     }
     for (int b0 = 0; b0 < batch; b0 += chunk) {
         const int cb = std::min(chunk, batch - b0);
@@ -1030,21 +834,12 @@ void tc_product(cudaStream_t st, int m, int n, int k, int batch, const zc* A, in
             ++launch_count();
         }
         if (!b_bcast) {
-            tc_split_b_kernel<<<(unsigned)((cb * (long long)n * 32 + 127) / 128), 128, 0, st>>>(
-                n, k, Kp, S, cb, B ? B + (long long)b0 * b_stride : nullptr, Br ? Br + (long long)b0 * b_stride : nullptr,
-                ldb, b_stride, pb, deb + (long long)b0 * n);
-            ++launch_count();
+            split_b(st, n, k, Kp, S, cb, B ? B + (long long)b0 * b_stride : nullptr, Br ? Br + (long long)b0 * b_stride : nullptr, ldb,
+                    b_stride, pb, deb + (long long)b0 * n);
         }
-        if (resident) {
-            const dim3 grid((n + kTileNr - 1) / kTileNr, (2 * m + kTileM - 1) / kTileM, cb);
-            tc_gemm_resident_kernel<<<grid, kThreads, smem_bytes, st>>>(map_a, map_b, S, plan.s0, Kp / kTileK, m, n, b0,
-                                                                        a_bcast, b_bcast, dea, deb, C0, c0_stride, C, ldc,
-                                                                        c_stride, s_ab, s_c, skip, skip_value, err);
-        } else {
-            const dim3 grid((n + kTileN - 1) / kTileN, (2 * m + kTileM - 1) / kTileM, cb);
-            tc_gemm_kernel<<<grid, kThreads, smem_bytes, st>>>(map_a, map_b, plan, m, n, b0, a_bcast, b_bcast, dea, deb, C0,
-                                                               c0_stride, C, ldc, c_stride, s_ab, s_c, skip, skip_value, err);
-        }
+        const dim3 grid((n + kTileN - 1) / kTileN, (2 * m + kTileM - 1) / kTileM, cb);
+        tc_gemm_kernel<<<grid, kThreads, smem_bytes, st>>>(map_a, map_b, plan, m, n, b0, a_bcast, b_bcast, dea, deb, C0,
+                                                           c0_stride, C, ldc, c_stride, s_ab, s_c, skip, skip_value, err);
         ++launch_count();
         RCWA_CUDA(cudaGetLastError());
     }
