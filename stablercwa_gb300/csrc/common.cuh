@@ -135,6 +135,18 @@ __device__ __forceinline__ zc ldz(const zc* p) {
 }
 __device__ __forceinline__ void stz(zc* p, zc v) { *reinterpret_cast<double2*>(p) = make_double2(v.re, v.im); }
 
+// a b + c as one 32 x 32 + 64 multiply-add (written out: from a mix of signed limbs and masked 64-bit values the
+// compiler forms 64 x 64 products, three instructions each)
+__device__ __forceinline__ long long fix_mad(int a, int b, long long c) {
+#ifdef __CUDA_ARCH__
+    long long r;
+    asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(c));
+    return r;
+#else
+    return (long long)a * b + c;
+#endif
+}
+
 // Right-hand side forms of the batched solve.
 enum RhsKind : int { RHS_DENSE = 0, RHS_IDENTITY = 1, RHS_DIAG = 2 };
 

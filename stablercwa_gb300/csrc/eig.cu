@@ -147,8 +147,8 @@ long long take_rotation_count() {
     return (long long)h;
 }
 
-// Hermitian matrices: the tridiagonalisation with G lanes per matrix, the QL iteration one lane per matrix,
-// the rotations applied row-parallel, and the fused kernel for any matrix whose rotation log overflowed.
+// Hermitian matrices: the tridiagonalisation with G lanes per matrix (small batches: fixed point, a CTA per matrix),
+// the QL iteration one lane per matrix (fixed point with the default settings), the rotations applied row-parallel, and the fused kernel for any matrix whose rotation log overflowed.
 // While 32 rows of the real rotation product fit in shared memory (n <= 904) the rotations go to a real
 // identity Y, in fixed point on the integer pipes, and the eigenvectors are Q Y; otherwise they are applied
 // to the complex Q in place in FP64.
@@ -260,6 +260,13 @@ bool herm_blocked_wanted(int n, int group) {
     return group <= 32 && n >= 64 && tc_gemm_enabled() && !Fp64ProductsGuard::active();
 }
 
+// The fixed-point reduction (a CTA per matrix) against the FP64 ones (lane groups, blocked from order 64; a CTA for
+// few matrices), whole eigensolves in ms: order 121: 1 matrix 14.2 / 20.2, 304 23.2 / 28.6, 608 35.4 / 34.2, 4096
+// 170 / 127; order 301: 1 88 / 193, 152 225 / 283, 304 390 / 289; order 161: 304 54 / 59, 1000 137 / 94; order 61:
+// 1 4.2 / 5.8, 1000 10.1 / 11.0; order 41: 1 2.0 / 2.7, 4000 12.5 / 10.5. The line lies where n * batch matrices'
+// columns fill the GPU's SMs about three deep.
+bool herm_fixed_reduce_wanted(int n, int batch) { return (long long)n * batch <= 48000 && eig_fixed_possible(n); }
+
 void herm_fused_dispatch(cudaStream_t st, int n, int batch, const zc* a, long long a_stride, zc* w, zc* v, int* info,
                          zc* ws, double eps, int max_iter, int group, const int* only) {
     const int tpb = 128;
@@ -286,14 +293,19 @@ void launch_eig_herm(cudaStream_t st, int n, int batch, const zc* a, long long a
         if (autotune_wanted(1, n, batch)) autotune_eig(st, 1, n, batch, a, a_stride, nullptr);
         group = tuned_eig_form(1, n, batch);
     }
+    // fixed point (eig_fixed.cuh) with the default settings: the QL iteration always, the reduction where no FP64
+    // form is forced or recorded and the batch is small (herm_fixed_reduce_wanted)
+    const bool fixed = eps == DBL_EPSILON && max_iter >= 30 && eig_fixed_enabled();
+    const bool fixed_reduce = fixed && group == 0 && herm_fixed_reduce_wanted(n, batch);
     if (group <= 0) group = eig_default_group(n, batch);
     TimedLaunch timed(TK_EIG, st);
     const size_t ysm = (size_t)n * kHermRows * sizeof(double);
     const bool real_form = ysm + kHermApplyStaticSmem <= 227 * 1024;
     zc* q = v;
     double* y = nullptr;
-    const bool blocked = real_form && herm_blocked_wanted(n, group);
+    const bool blocked = !fixed_reduce && real_form && herm_blocked_wanted(n, group);
     zc *pan = nullptr, *mall = nullptr, *u = nullptr;
+    int* status = nullptr;  // matrices the fixed-point reduction left to the fused kernel
     if (real_form) {
         RCWA_CUDA(cudaMallocAsync(&q, (size_t)batch * n * n * sizeof(zc), st));  // Q, or the reflectors when blocked
         RCWA_CUDA(cudaMallocAsync(&y, (size_t)batch * n * n * sizeof(double), st));
@@ -304,6 +316,9 @@ void launch_eig_herm(cudaStream_t st, int n, int batch, const zc* a, long long a
         RCWA_CUDA(cudaMallocAsync(&mall, (size_t)batch * pnb * n * sizeof(zc), st));
         RCWA_CUDA(cudaMallocAsync(&u, (size_t)batch * kHermNb * n * sizeof(zc), st));
         herm_blocked_reduce(st, n, batch, a, a_stride, ws, pan, q, mall, group);
+    } else if (fixed_reduce) {
+        RCWA_CUDA(cudaMallocAsync(&status, (size_t)batch * sizeof(int), st));
+        launch_herm_reduce_fixed(st, n, batch, a, a_stride, q, ws, status);
     } else {
         herm_reduce_dispatch(st, n, batch, a, a_stride, q, ws, group);
     }
@@ -316,6 +331,8 @@ void launch_eig_herm(cudaStream_t st, int n, int batch, const zc* a, long long a
             case 16: herm_dc_launch<16>(st, n, batch, ws, y, w, info, eps, max_iter); break;
             default: herm_dc_launch<32>(st, n, batch, ws, y, w, info, eps, max_iter); break;
         }
+    } else if (fixed && real_form && qsm <= 227 * 1024) {
+        launch_herm_ql_fixed(st, n, batch, w, info, ws, status);
     } else if (qsm <= 227 * 1024) {
         if (qsm > 48 * 1024) ensure_smem_optin(reinterpret_cast<const void*>(herm_ql_kernel<true, true>), (int)qsm);
         // the real form's log is fixed point (herm_apply_real_kernel); the shared-memory form implies it
@@ -356,6 +373,7 @@ void launch_eig_herm(cudaStream_t st, int n, int batch, const zc* a, long long a
     }
     herm_fused_dispatch(st, n, batch, a, a_stride, w, v, info, ws, eps, max_iter, group, only);
     RCWA_CUDA(cudaFreeAsync(only, st));
+    if (status) RCWA_CUDA(cudaFreeAsync(status, st));
     if (real_form) {
         RCWA_CUDA(cudaFreeAsync(q, st));
         RCWA_CUDA(cudaFreeAsync(y, st));

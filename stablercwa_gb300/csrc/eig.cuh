@@ -1675,7 +1675,7 @@ static __global__ void __launch_bounds__(kHermRows) herm_apply_real_kernel(int n
         long long pos = 0;
         for (int k = 0; k < sweeps; ++k) {
             const int2 fl = table[k];
-            long long cur = y[(fl.y + 1) * kHermRows];
+            long long cur = y[(fl.y + 1) * kHermRows], yn = y[fl.y * kHermRows];
             for (int i = fl.y; i >= fl.x; --i, ++pos) {
                 if (pos == cb + kHermRows) {  // the next chunk: stage it, start loading the one after
                     stage[b ^ 1][t] = next;
@@ -1686,17 +1686,19 @@ static __global__ void __launch_bounds__(kHermRows) herm_apply_real_kernel(int n
                     __syncwarp();
                 }
                 const int4 e = stage[b][pos - cb];
-                const long long yi = y[i * kHermRows];
+                const long long yi = yn;
+                yn = y[(i > fl.x ? i - 1 : fl.x) * kHermRows];  // ahead of its rotation
                 const int a1 = (int)(yi >> 31), a0 = (int)(yi & 0x7fffffff);
                 const int b1 = (int)(cur >> 31), b0 = (int)(cur & 0x7fffffff);
                 // the y_i terms first: they do not wait for the previous rotation's output
-                long long u1 = (long long)e.x * a0 + (long long)e.y * a1 + (1LL << 30);
-                long long u2 = (long long)e.z * -a0 + (long long)e.w * -a1 + (1LL << 30);
-                const long long v1 = (long long)e.x * a1, v2 = (long long)e.z * -a1;
-                u1 += (long long)e.z * -b0 + (long long)e.w * -b1;
-                u2 += (long long)e.x * -b0 + (long long)e.y * -b1;
-                y[(i + 1) * kHermRows] = v1 + (long long)e.z * -b1 + (u1 >> 31);
-                cur = v2 + (long long)e.x * -b1 + (u2 >> 31);
+                const long long half = 1LL << 30;
+                long long u1 = fix_mad(e.y, a1, fix_mad(e.x, a0, half));
+                long long u2 = fix_mad(e.w, -a1, fix_mad(e.z, -a0, half));
+                const long long v1 = fix_mad(e.x, a1, 0), v2 = fix_mad(e.z, -a1, 0);
+                u1 = fix_mad(e.w, -b1, fix_mad(e.z, -b0, u1));
+                u2 = fix_mad(e.y, -b1, fix_mad(e.x, -b0, u2));
+                y[(i + 1) * kHermRows] = fix_mad(e.z, -b1, v1) + (u1 >> 31);
+                cur = fix_mad(e.x, -b1, v2) + (u2 >> 31);
             }
             y[fl.x * kHermRows] = cur;
         }

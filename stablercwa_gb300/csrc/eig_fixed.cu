@@ -17,7 +17,14 @@ constexpr int kFixMinOrder = 24;
 constexpr int kFixPassMin = 456;
 constexpr long long kFixLogBytes = 4LL << 30;
 
-bool fix_enabled() {
+// warps of fix_schur_kernel's CTA: a lane per row or column of the matrix up to order 352 (11 warps' tiles are
+// what shared memory holds), at least four so that three warps trail the one that forms the rotations
+int fix_warps(int n) { return std::min(11, std::max(4, (n + 31) / 32)); }
+
+}  // namespace
+
+// RCWA_GB300_EIG_FIXED=0 keeps the FP64 iterations
+bool eig_fixed_enabled() {
     static const bool on = [] {
         const char* e = std::getenv("RCWA_GB300_EIG_FIXED");
         return !(e && e[0] == '0');
@@ -25,13 +32,7 @@ bool fix_enabled() {
     return on;
 }
 
-// warps of fix_schur_kernel's CTA: a lane per row or column of the matrix up to order 352 (11 warps' tiles are
-// what shared memory holds), at least four so that three warps trail the one that forms the rotations
-int fix_warps(int n) { return std::min(11, std::max(4, (n + 31) / 32)); }
-
-}  // namespace
-
-bool eig_fixed_possible(int n) { return fix_enabled() && n >= kFixMinOrder && n <= kFixMaxOrder; }
+bool eig_fixed_possible(int n) { return eig_fixed_enabled() && n >= kFixMinOrder && n <= kFixMaxOrder; }
 
 long long eig_fixed_bytes(int n) {
     if (!eig_fixed_possible(n)) return 0;
@@ -44,8 +45,8 @@ void launch_eig_fixed(cudaStream_t st, int n, int batch, const zc* a, long long 
     const int warps = fix_warps(n);
     const size_t schur_smem = fix_schur_smem(n, warps), row_smem = (size_t)n * 32 * sizeof(lz),
                  back_smem = (size_t)(n + 4) * 32 * sizeof(zc);
-    ensure_smem_optin(reinterpret_cast<const void*>(fix_schur_kernel), (int)schur_smem);
-    if (row_smem > 46 * 1024) ensure_smem_optin(reinterpret_cast<const void*>(fix_apply_kernel), (int)row_smem);
+    ensure_smem_optin(reinterpret_cast<const void*>(fix_schur_kernel<false>), (int)schur_smem);
+    if (row_smem > 45 * 1024) ensure_smem_optin(reinterpret_cast<const void*>(fix_apply_kernel), (int)row_smem);
     if (back_smem > 48 * 1024) ensure_smem_optin(reinterpret_cast<const void*>(fix_backsub_kernel), (int)back_smem);
     const int chunk = (int)std::max(1LL, std::min<long long>(std::min(batch, std::max(kFixPassMin, (batch + 1) / 2)),
                                                              kFixLogBytes / eig_fixed_bytes(n)));
@@ -63,10 +64,11 @@ void launch_eig_fixed(cudaStream_t st, int n, int batch, const zc* a, long long 
         zc *wc = w + (long long)b0 * n, *vc = v + (long long)b0 * nn, *wsc = ws + (long long)b0 * wst;
         zc *z1 = wsc + nn, *z2 = wsc + 2 * nn;  // Z; X
         lz* h = reinterpret_cast<lz*>(wsc);
-        fix_schur_kernel<<<(unsigned)cb, 32 * warps, schur_smem, st>>>(n, cb, ac, a_stride, wc, h, wst, log, table, head, status,
+        fix_schur_kernel<false><<<(unsigned)cb, 32 * warps, schur_smem, st>>>(n, cb, ac, a_stride, wc, h, wst, log, 2 * fix_log_capacity(n), table, head, status,
                                                                        done + b0, info + b0);
         RCWA_CUDA(cudaGetLastError());
-        fix_apply_kernel<<<dim3((unsigned)cb, (unsigned)((n + 31) / 32)), 32, row_smem, st>>>(n, cb, z1, wst, log, table, head, status);
+        fix_apply_kernel<<<dim3((unsigned)cb, (unsigned)((n + 31) / 32)), 32, row_smem, st>>>(n, cb, z1, wst, log, 2 * fix_log_capacity(n), table,
+                                                                                               head, status);
         RCWA_CUDA(cudaGetLastError());
         zc* t = t_out ? t_out + (long long)b0 * nn : vc;
         RCWA_CUDA(cudaMemsetAsync(tn, 0, (size_t)cb * sizeof(unsigned long long), st));
@@ -86,6 +88,37 @@ void launch_eig_fixed(cudaStream_t st, int n, int batch, const zc* a, long long 
         launch_count() += 2;
     }
     for (void* p : {(void*)log, (void*)table, (void*)head, (void*)status, (void*)tn}) RCWA_CUDA(cudaFreeAsync(p, st));
+}
+
+// The Hermitian solver's reduction: d and e into ws (where the QL kernel reads them) and Q (n x n, contiguous);
+// status[b] = 1 for a matrix left to the FP64 kernels.
+void launch_herm_reduce_fixed(cudaStream_t st, int n, int batch, const zc* a, long long a_stride, zc* q, zc* ws, int* status) {
+    const long long nn = (long long)n * n, wst = 3 * nn + 4LL * n + 8, log_stride = 2 * fix_reduce_capacity(n);
+    const int warps = fix_warps(n);
+    const size_t schur_smem = fix_schur_smem(n, warps), row_smem = (size_t)n * 32 * sizeof(lz);
+    ensure_smem_optin(reinterpret_cast<const void*>(fix_schur_kernel<true>), (int)schur_smem);
+    if (row_smem > 45 * 1024) ensure_smem_optin(reinterpret_cast<const void*>(fix_apply_kernel), (int)row_smem);
+    int4* log = nullptr;
+    int* head = nullptr;
+    RCWA_CUDA(cudaMallocAsync(&log, (size_t)batch * log_stride * sizeof(int4), st));
+    RCWA_CUDA(cudaMallocAsync(&head, (size_t)batch * 2 * sizeof(int), st));
+    fix_schur_kernel<true><<<(unsigned)batch, 32 * warps, schur_smem, st>>>(n, batch, a, a_stride, nullptr, reinterpret_cast<lz*>(ws), wst,
+                                                                            log, log_stride, nullptr, head, status, nullptr, nullptr);
+    RCWA_CUDA(cudaGetLastError());
+    fix_apply_kernel<<<dim3((unsigned)batch, (unsigned)((n + 31) / 32)), 32, row_smem, st>>>(n, batch, q, nn, log, log_stride, nullptr, head,
+                                                                                             status);
+    RCWA_CUDA(cudaGetLastError());
+    launch_count() += 2;
+    RCWA_CUDA(cudaFreeAsync(log, st));
+    RCWA_CUDA(cudaFreeAsync(head, st));
+}
+
+void launch_herm_ql_fixed(cudaStream_t st, int n, int batch, zc* w, int* info, zc* ws, const int* status) {
+    const size_t smem = (size_t)2 * n * kHermQlThreads * sizeof(long long);
+    if (smem > 48 * 1024) ensure_smem_optin(reinterpret_cast<const void*>(herm_ql_fixed_kernel), (int)smem);
+    herm_ql_fixed_kernel<<<(unsigned)((batch + kHermQlThreads - 1) / kHermQlThreads), kHermQlThreads, smem, st>>>(
+        n, batch, w, info, ws, status, rotation_counter());
+    RCWA_CUDA(cudaGetLastError());
 }
 
 }  // namespace rcwa_gb300

@@ -33,7 +33,7 @@
 // Sums that a later sweep needs exactly (H - t) are exact: shifts are integers.
 #pragma once
 
-#include "common.cuh"
+#include "eig.cuh"
 
 namespace rcwa_gb300 {
 
@@ -53,7 +53,8 @@ constexpr int kFixEntry = 3;         // int4s of a rotation in shared memory (tw
 // log capacity in rotations: the reduction's (n^2 / 2 and a phase per segment) and 2.5 n^2 of the QR sweeps (a
 // random matrix takes about 1.8 n^2, a grating layer's 1.0 n^2; a matrix that would need more is left to the
 // FP64 kernels)
-__host__ __device__ inline long long fix_log_capacity(int n) { return (long long)n * n / 2 + 17LL * n + 160 + 5LL * n * n / 2; }
+__host__ __device__ inline long long fix_reduce_capacity(int n) { return (long long)n * n / 2 + 17LL * n + 160; }
+__host__ __device__ inline long long fix_log_capacity(int n) { return fix_reduce_capacity(n) + 5LL * n * n / 2; }
 __host__ __device__ inline long long fix_table_capacity(int n) { return 8LL * n + 64; }
 // shared memory of fix_schur_kernel: a tile a warp, one column's or sweep's rotations, the diagonal, the
 // subdiagonal, the sweep's phase, reduction slots
@@ -64,18 +65,6 @@ __host__ __device__ inline size_t fix_schur_smem(int n, int warps) {
 __device__ __forceinline__ void fix_limbs(long long c, int& hi, int& lo) {
     lo = (int)((unsigned)c << 2) >> 2;
     hi = (int)(c >> 30) + (int)(((unsigned)c >> 29) & 1u);
-}
-
-// a b + c as one 32 x 32 + 64 multiply-add (written out: from a mix of signed limbs and masked 64-bit values the
-// compiler forms 64 x 64 products, three instructions each)
-__device__ __forceinline__ long long fix_mad(int a, int b, long long c) {
-#ifdef __CUDA_ARCH__
-    long long r;
-    asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(c));
-    return r;
-#else
-    return (long long)a * b + c;
-#endif
 }
 
 // an entry's component as limbs y1 2^30 + y0 (|y| < 2^61)
@@ -131,32 +120,15 @@ __device__ __forceinline__ float fix_rsqrt(float x) {
 #endif
 }
 
-// The rotation that takes (x, sub) to (nrm, 0): q = x / nrm, s = sub / nrm, nrm^2 = |x|^2 + sub^2; the
-// identity for x = sub = 0. |components| < 2^61.
-__device__ __forceinline__ FixRot fix_rotation(long long xr, long long xi, long long sub) {
-    int h;
-    const auto tops = [&] {
-        const int a = (int)(xr >> 32), b = (int)(xi >> 32), c = (int)(sub >> 32);
-        h = (a ^ (a >> 31)) | (b ^ (b >> 31)) | (c ^ (c >> 31));
-    };
-    tops();
-    if (h == 0) {  // all of them below 2^32 units
-        if ((xr | xi | sub) == 0) xr = 1;
-        xr <<= 27;
-        xi <<= 27;
-        sub <<= 27;
-        tops();
-        if (h == 0) {
-            xr <<= 27;
-            xi <<= 27;
-            sub <<= 27;
-            tops();
-        }
-    }
-    const int sh = __clz(h) - 3;  // the largest into [2^60, 2^61)
-    xr <<= sh;
-    xi <<= sh;
-    sub <<= sh;
+// the high words of |.| of three values (up to their signs' one unit), together
+__device__ __forceinline__ int fix_tops(long long x, long long y, long long z) {
+    const int a = (int)(x >> 32), b = (int)(y >> 32), c = (int)(z >> 32);
+    return (a ^ (a >> 31)) | (b ^ (b >> 31)) | (c ^ (c >> 31));
+}
+
+// The rotation that takes (x, sub) to (nrm, 0): q = x / nrm, s = sub / nrm, nrm^2 = |x|^2 + sub^2, from components
+// scaled so that the largest magnitude is in [2^60, 2^61).
+__device__ __forceinline__ FixRot fix_rotation_scaled(long long xr, long long xi, long long sub) {
     const FixLimb a = fix_split(xr), b = fix_split(xi), c = fix_split(sub);
     // Q = (a^2 + b^2 + c^2) 2^-60, in [2^60, 3 2^62) (unsigned); + 1: the dropped squares of the low limbs on average
     long long u = fix_mad(a.h, a.l, 1LL << 28);
@@ -192,6 +164,26 @@ __device__ __forceinline__ FixRot fix_rotation(long long xr, long long xi, long 
     r.ns1 = -r.s1;
     r.ns0 = -r.s0;
     return r;
+}
+
+// The same from components below 2^61; the identity for x = sub = 0.
+__device__ __forceinline__ FixRot fix_rotation(long long xr, long long xi, long long sub) {
+    int h = fix_tops(xr, xi, sub);
+    if (h == 0) {  // all of them below 2^32 units
+        if ((xr | xi | sub) == 0) xr = 1;
+        xr <<= 27;
+        xi <<= 27;
+        sub <<= 27;
+        h = fix_tops(xr, xi, sub);
+        if (h == 0) {
+            xr <<= 27;
+            xi <<= 27;
+            sub <<= 27;
+            h = fix_tops(xr, xi, sub);
+        }
+    }
+    const int sh = __clz(h) - 3;  // the largest into [2^60, 2^61)
+    return fix_rotation_scaled(xr << sh, xi << sh, sub << sh);
 }
 
 // a rotation in shared memory (kFixEntry int4s) and in the log (two)
@@ -292,12 +284,14 @@ __device__ __forceinline__ lz fix_left_block(int n, lz* H, lz* tile, const int4*
 
 constexpr int kFixBatch = 6;  // columns whose entries a row's lane holds at once, and as many on their way
 
-// Schur reduction of one matrix. H: n x n lz (column-major, global). log: rotations (two int4 each), table:
+// Schur reduction of one matrix; with Herm only step 1, on the Hermitian part (A + A^H) / 2: the reduced matrix is
+// real symmetric tridiagonal, its d and e go where the QL kernel reads them. H: n x n lz (column-major, global). log: rotations (two int4 each), table:
 // (l, en, phase) per sweep in int4. w: eigenvalues in deflation order. status: 0 done, 1 left to the FP64
 // kernels (non-finite input, no convergence, log full). head: the
 // number of sweeps and the exponent of the unit.
-static __global__ void fix_schur_kernel(int n, int batch, const zc* __restrict__ a_in, long long a_stride, zc* __restrict__ w_out,
-                                        lz* __restrict__ h_ws, long long h_stride, int4* __restrict__ log_all,
+template <bool Herm>
+__global__ void fix_schur_kernel(int n, int batch, const zc* __restrict__ a_in, long long a_stride, zc* __restrict__ w_out,
+                                        lz* __restrict__ h_ws, long long h_stride, int4* __restrict__ log_all, long long log_stride,
                                         int4* __restrict__ table_all, int* __restrict__ head, int* __restrict__ status,
                                         int* __restrict__ done, int* __restrict__ info) {
     RCWA_DYN_SMEM(lz, fix_sm);
@@ -313,7 +307,7 @@ static __global__ void fix_schur_kernel(int n, int batch, const zc* __restrict__
     int* flags = reinterpret_cast<int*>(sub + n);                           // 48 reduction slots, [48] the phase flag
     const zc* A = a_in + gid * a_stride;
     lz* H = h_ws + gid * h_stride;
-    int4* log = log_all + 2 * gid * fix_log_capacity(n);
+    int4* log = log_all + gid * log_stride;
     int4* table = table_all + gid * fix_table_capacity(n);
     const long long nn = (long long)n * n;
     const lz zero{0, 0};
@@ -334,7 +328,7 @@ static __global__ void fix_schur_kernel(int n, int batch, const zc* __restrict__
     if (top < 200 || top > 1900) {
         if (tid == 0) {
             status[gid] = 1;
-            done[gid] = 0;
+            if (!Herm) done[gid] = 0;
         }
         return;
     }
@@ -382,7 +376,15 @@ static __global__ void fix_schur_kernel(int n, int batch, const zc* __restrict__
     }
     // N = 2^(top - 1023) min(..) < 2^(e2 + kFixNormBits)
     const int e2 = ((__float_as_int(fminf(sqrtf(ss), sqrtf(rmax * cmax)) * 1.001f) >> 23) & 0xff) - 127 + 1 + (top - 1023) - kFixNormBits;
-    for (long long i = tid; i < nn; i += nthr) H[i] = lz{fix_from_double(A[i].re, e2), fix_from_double(A[i].im, e2)};
+    if constexpr (Herm) {
+        for (long long i = tid; i < nn; i += nthr) {
+            const int c = (int)(i / n), r = (int)(i - (long long)c * n);
+            const zc x = A[i], y = A[(long long)r * n + c];
+            H[i] = lz{fix_from_double(0.5 * (x.re + y.re), e2), fix_from_double(0.5 * (x.im - y.im), e2)};
+        }
+    } else {
+        for (long long i = tid; i < nn; i += nthr) H[i] = lz{fix_from_double(A[i].re, e2), fix_from_double(A[i].im, e2)};
+    }
     __syncthreads();
 
     // ---- Hessenberg form
@@ -526,8 +528,22 @@ static __global__ void fix_schur_kernel(int n, int batch, const zc* __restrict__
     if (tid == 0) sub[0] = 0;
     __syncthreads();
 
+    if constexpr (Herm) {
+        const double unit = __longlong_as_double((long long)(e2 + 1023) << 52);
+        double* d = reinterpret_cast<double*>(H + 2 * nn);
+        for (int i = tid; i < n; i += nthr) {
+            d[i] = (double)dg[i].re * unit;
+            d[n + i] = i + 1 < n ? (double)sub[i + 1] * unit : 0.0;
+        }
+        if (tid == 0) {
+            head[2 * gid] = 0;
+            status[gid] = 0;
+        }
+        return;
+    }
+
     // ---- shifted QR
-    const long long log_cap = fix_log_capacity(n), tab_cap = fix_table_capacity(n);
+    const long long log_cap = log_stride / 2, tab_cap = fix_table_capacity(n);
     const double unit = __longlong_as_double((long long)(e2 + 1023) << 52);
     lz t{0, 0};
     int en = n - 1, its = 0, sweeps = 0, fail = 0;
@@ -753,8 +769,8 @@ static __global__ void fix_schur_kernel(int n, int batch, const zc* __restrict__
 // Z from the log: a lane per row, 32 rows a CTA, the row in shared memory (row t of the CTA at element
 // i * 32 + t). A similarity H <- G H G^H takes Z <- Z G^H: (a', b') = (q a + s b, conj(q) b - s a).
 static __global__ void __launch_bounds__(32) fix_apply_kernel(int n, int batch, zc* __restrict__ z_out, long long z_stride,
-                                                              const int4* __restrict__ log_all, const int4* __restrict__ table_all,
-                                                              const int* __restrict__ head, const int* __restrict__ status) {
+                                                              const int4* __restrict__ log_all, long long log_stride,
+                                                              const int4* __restrict__ table_all, const int* __restrict__ head, const int* __restrict__ status) {
     RCWA_DYN_SMEM(lz, fixz_sm);
     const long long gid = blockIdx.x;
     const int lane = threadIdx.x, row = blockIdx.y * 32 + lane;
@@ -764,7 +780,7 @@ static __global__ void __launch_bounds__(32) fix_apply_kernel(int n, int batch, 
     // the log through shared memory: chunk c (32 rotations) in stage[c & 1], the next in registers on its way.
     // Runs of rotations are cut at the chunks' ends, so that nothing inside a run depends on the staging.
     __shared__ int4 stage[2][68];  // a run reads one rotation past its end
-    const int4* log = log_all + 2 * gid * fix_log_capacity(n) + lane;
+    const int4* log = log_all + gid * log_stride + lane;
     const int4* table = table_all + gid * fix_table_capacity(n);
     stage[0][lane] = log[0];
     stage[0][lane + 32] = log[32];
@@ -959,6 +975,159 @@ static __global__ void __launch_bounds__(128) fix_unit_columns_kernel(int n, int
     ssq = group_sum<32>(ssq, 0xffffffffu);
     const double inv = 1.0 / sqrt(ssq);
     for (int r = lane; r < n; r += 32) c[r] = zdivr(c[r], big) * inv;
+}
+
+// ---------------------------------------------------------------- the Hermitian solver's QL iteration
+//
+// herm_ql_kernel's iteration (eig.cuh: implicit QL with Wilkinson's shift on d and e, one thread per matrix, every
+// rotation logged for herm_apply_real_kernel) in fixed point. Its chain of about 20 dependent FP64 instructions a
+// rotation, 64 cycles each, took 1.1 us (17.2 ms for one matrix of order 121); the same chain in integers takes
+// 0.5 us (7.4 ms), and 4096 matrices' 20 ms went to MEASURED_Q. d and e are scaled so that
+// N >= ||T||_2 (Gershgorin's bound) lies in [2^58, 2^59) units: the iteration's quantities stay below 4 N. What it does
+// not finish (non-finite or zero matrices, scales whose powers of two are not normal doubles, 30 sweeps without a
+// deflation) is flagged as a full log is, for the fused FP64 kernel. status, if given: matrices whose reduction left
+// them to that kernel already.
+constexpr int kFixQlBits = 59;
+static __global__ void __launch_bounds__(kHermQlThreads) herm_ql_fixed_kernel(int n, int batch, zc* __restrict__ w,
+                                                                             int* __restrict__ info, zc* __restrict__ ws,
+                                                                             const int* __restrict__ status,
+                                                                             unsigned long long* rotations) {
+    RCWA_DYN_SMEM(long long, fixq_sm);
+    const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (gid >= batch) return;
+    zc* base = ws + gid * eig_workspace_elems(n);
+    const double* src = reinterpret_cast<const double*>(base + 2LL * n * n);
+    int* tail = reinterpret_cast<int*>(base + 3LL * n * n);  // [0] sweeps, [1] left to the fused kernel
+    long long* d = fixq_sm + threadIdx.x;
+    long long* e = d + (long long)n * kHermQlThreads;
+    constexpr int sd = kHermQlThreads;
+    // the scale
+    float big = 0.0f;
+    int e2 = 0;
+    bool usable = !(status && status[gid]);
+    if (usable) {
+        int top = 0;
+        for (int k = 0; k < 2 * n; ++k) top = max(top, (int)((__double_as_longlong(src[k]) >> 52) & 0x7FF));
+        usable = top >= 200 && top <= 1900;
+        if (usable) {
+            const double scl = __longlong_as_double((long long)(2046 - top) << 52);
+            float below = 0.0f;
+            for (int k = 0; k < n; ++k) {
+                const float ek = k + 1 < n ? fabsf((float)(src[n + k] * scl)) : 0.0f;
+                big = fmaxf(big, fabsf((float)(src[k] * scl)) + ek + below);
+                below = ek;
+            }
+            e2 = ((__float_as_int(big * 1.001f) >> 23) & 0xff) - 127 + 1 + (top - 1023) - kFixQlBits;
+        }
+    }
+    tail[0] = 0;
+    tail[1] = !usable;
+    info[gid] = 0;
+    if (!usable) return;
+    for (int k = 0; k < n; ++k) {
+        d[k * sd] = fix_from_double(src[k], e2);
+        e[k * sd] = k + 1 < n ? fix_from_double(src[n + k], e2) : 0;
+    }
+    int2* table = reinterpret_cast<int2*>(reinterpret_cast<double*>(base) + 2 * n);
+    int4* log = reinterpret_cast<int4*>(base + (long long)n * n);
+    const long long log_cap = herm_log_capacity(n), table_cap = herm_table_capacity(n);
+    long long pos = 0, sweeps = 0;
+    bool left = false;
+    for (int l = 0; l < n && !left; ++l) {
+        for (int its = 0;; ++its) {
+            // first m >= l with e[m] below eps (|d[m]| + |d[m+1]|), or of two units (2^-57 N at most)
+            int m = l;
+            for (; m < n - 1; ++m) {
+                const long long a = d[m * sd], b = d[(m + 1) * sd], x = e[m * sd];
+                const unsigned long long size = (unsigned long long)((a < 0 ? -a : a) + (b < 0 ? -b : b));
+                const unsigned long long ax = (unsigned long long)(x < 0 ? -x : x);
+                if (ax <= 2 || ax <= size >> 52) break;
+            }
+            if (m == l) break;
+            if (its == 30 || pos + (m - l) > log_cap || sweeps + 1 > table_cap) {
+                left = true;
+                break;
+            }
+            // g = d[m] - shift, the shift d[l] - e^2 / (h + sign(h) sqrt(h^2 + e^2)), h = (d[l+1] - d[l]) / 2, its
+            // correction in float
+            long long g = d[m * sd] - d[l * sd];
+            {
+                const float k = 0x1p-59f;
+                const float h = (float)((d[(l + 1) * sd] - d[l * sd]) >> 1) * k, x = (float)e[l * sd] * k;
+                const float den = h + copysignf(sqrtf(h * h + x * x), h);
+                if (fabsf(den) > 1e-18f) g += (long long)(x * (x / den) * 0x1p59f);
+            }
+            FixRot q;  // c and s of the last rotation (c in q.cr, s in q.s)
+            q.cr1 = q.s1 = 1 << 30;
+            q.cr0 = q.s0 = 0;
+            long long p = 0;
+            bool split = false;
+            int i = m - 1;
+            long long ei = e[i * sd], di = d[i * sd], dn = d[m * sd];
+            for (; i >= l; --i) {
+                const FixLimb el = fix_split(ei), o{0, 0};
+                const long long b = fix_dot3(0, 0, o, 0, 0, o, q.cr1, q.cr0, el);
+                // f = s e exactly, 60 fractional bits in fl: where f and g are both small the angle between them,
+                // which carries the shift up the matrix, needs f's digits below one unit
+                const long long ll = fix_mad(q.s0, el.l, 0), u = fix_mad(q.s0, el.h, fix_mad(q.s1, el.l, ll >> 30));
+                const long long f = fix_mad(q.s1, el.h, u >> 30);
+                const unsigned long long fl = (unsigned long long)((unsigned)u & 0x3fffffffu) << 30 | ((unsigned)ll & 0x3fffffffu);
+                // the next rotation's entries, ahead of their use
+                const int in = i > l ? i - 1 : l;
+                const long long en = e[in * sd], dp = d[in * sd];
+                if (f == 0 && fl == 0 && g == 0) {
+                    e[(i + 1) * sd] = 0;
+                    d[(i + 1) * sd] = dn - p;
+                    e[m * sd] = 0;
+                    split = true;
+                    break;
+                }
+                {
+                    long long x = g, y = f;
+                    unsigned long long r = fl;
+                    int h = fix_tops(x, y, 0);
+                    while (h == 0) {
+                        x <<= 28;
+                        y = y << 28 | (long long)(r >> 32);
+                        r = (r << 28) & 0xfffffffffffffffull;
+                        h = fix_tops(x, y, 0);
+                    }
+                    const int sh = __clz(h) - 3;
+                    q = fix_rotation_scaled(x << sh, 0, y << sh | (long long)(r >> (60 - sh)));
+                }
+                e[(i + 1) * sd] = fix_dot3(0, 0, o, q.s1, q.s0, fix_split(f), q.cr1, q.cr0, fix_split(g));
+                const long long g2 = dn - p;
+                const long long t = fix_dot3(0, 0, o, q.cr1, q.cr0, fix_split(2 * b), q.s1, q.s0, fix_split(di - g2));
+                const FixLimb tl = fix_split(t);
+                p = fix_dot3(0, 0, o, 0, 0, o, q.s1, q.s0, tl);
+                d[(i + 1) * sd] = g2 + p;
+                g = fix_dot3(0, 0, o, 0, 0, o, q.cr1, q.cr0, tl) - b;
+                // the log's form (herm_fixed_entry): s 2^62 and -c 2^62 in 31-bit limbs, saturated below 2^62
+                const long long s62 = min((((long long)q.s1 << 30) + q.s0) << 2, 0x3fffffffffffffffLL),
+                                c62 = min((((long long)q.cr1 << 30) + q.cr0) << 2, 0x3fffffffffffffffLL);
+                const long long S = max(s62, -0x3fffffffffffffffLL), C = -max(c62, -0x3fffffffffffffffLL);
+                log[pos] = make_int4((int)(S >> 31), (int)(S & 0x7fffffff), (int)(C >> 31), (int)(C & 0x7fffffff));
+                ++pos;
+                dn = di;
+                ei = en;
+                di = dp;
+            }
+            const int first = split ? i + 1 : l;
+            if (!split) {
+                d[l * sd] = dn - p;
+                e[l * sd] = g;
+                e[m * sd] = 0;
+            }
+            if (m - 1 >= first) table[sweeps++] = make_int2(first, m - 1);
+        }
+    }
+    tail[0] = (int)sweeps;
+    tail[1] = left;
+    if (!left) {
+        const double unit = __longlong_as_double((long long)(e2 + 1023) << 52);
+        for (int k = 0; k < n; ++k) w[gid * n + k] = zc{(double)d[k * sd] * unit, 0.0};
+        if (rotations) atomicAdd(rotations, (unsigned long long)pos);
+    }
 }
 
 }  // namespace rcwa_gb300

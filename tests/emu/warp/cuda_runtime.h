@@ -55,6 +55,7 @@ inline int __ffs(unsigned x) { return __builtin_ffs((int)x); }
 inline unsigned long long __umul64hi(unsigned long long a, unsigned long long b) {
     return (unsigned long long)(((unsigned __int128)a * b) >> 64);
 }
+inline double rsqrt(double x) { return 1.0 / std::sqrt(x); }
 inline float rsqrtf(float x) { return 1.0f / std::sqrt(x); }
 
 void emu_block_sync();
@@ -93,5 +94,10 @@ inline unsigned __ballot_sync(unsigned, int pred) {
 inline unsigned long long atomicMax(unsigned long long* p, unsigned long long v) {
     const unsigned long long o = *p;
     *p = std::max(o, v);
+    return o;
+}
+inline unsigned long long atomicAdd(unsigned long long* p, unsigned long long v) {
+    const unsigned long long o = *p;
+    *p += v;
     return o;
 }

@@ -111,7 +111,7 @@ static void solve(const char* name, int n, const M& a, int warps, int want_statu
     std::vector<zc> w(n), Z(nn);
     int head[2] = {0, 0}, status = -1, done = -1, info = -1;
     run_cta(32 * warps, fix_schur_smem(n, warps), [&] {
-        fix_schur_kernel(n, 1, a.data(), nn, w.data(), H.data(), nn, log.data(), table.data(), head, &status, &done, &info);
+        fix_schur_kernel<false>(n, 1, a.data(), nn, w.data(), H.data(), nn, log.data(), (long long)log.size(), table.data(), head, &status, &done, &info);
     });
     if (status != want_status || done != !status) {
         std::printf("FAIL %s n=%d: status %d done %d\n", name, n, status, done);
@@ -124,7 +124,7 @@ static void solve(const char* name, int n, const M& a, int warps, int want_statu
     }
     for (int by = 0; by * 32 < n; ++by) {
         blockIdx.y = by;
-        run_cta(32, (size_t)n * 32 * sizeof(lz), [&] { fix_apply_kernel(n, 1, Z.data(), nn, log.data(), table.data(), head, &status); });
+        run_cta(32, (size_t)n * 32 * sizeof(lz), [&] { fix_apply_kernel(n, 1, Z.data(), nn, log.data(), (long long)log.size(), table.data(), head, &status); });
     }
     blockIdx.y = 0;
     M Zh(nn);
@@ -168,6 +168,63 @@ static void solve(const char* name, int n, const M& a, int warps, int want_statu
     const bool ok = orth <= 1e-13 && schur <= 1e-13 && worst <= 1e-13;
     std::printf("%s %-22s n=%3d warps %d: sweeps %d rotations %.2f n^2, orthogonality %.1e, Schur residual %.1e, eigenpairs %.1e\n",
                 ok ? "pass" : "FAIL", name, n, warps, head[0], (double)rot / nn, orth, schur, worst);
+    failures += !ok;
+}
+
+// The Hermitian solver's pieces: the reduction to tridiagonal form, Q from its log, the QL kernel, its rotations on a
+// real identity (herm_apply_real_kernel), V = Q Y.
+static void solve_hermitian(const char* name, int n, const M& a, int warps, int want_left) {
+    const long long nn = (long long)n * n;
+    std::vector<zc> ws(eig_workspace_elems(n)), w(n), Q(nn);
+    std::vector<int4> log(2 * fix_reduce_capacity(n)), table(1);
+    std::vector<double> Y(nn);
+    int head[2] = {0, 0}, status = -1, info = -1;
+    unsigned long long rot = 0;
+    run_cta(32 * warps, fix_schur_smem(n, warps), [&] {
+        fix_schur_kernel<true>(n, 1, a.data(), nn, w.data(), reinterpret_cast<lz*>(ws.data()), 0, log.data(), (long long)log.size(), table.data(), head,
+                               &status, nullptr, nullptr);
+    });
+    run_cta(32, (size_t)2 * n * kHermQlThreads * 8, [&] { herm_ql_fixed_kernel(n, 1, w.data(), &info, ws.data(), &status, &rot); });
+    const int left = reinterpret_cast<const int*>(ws.data() + 3 * nn)[1];
+    if (left != want_left || info != 0) {
+        std::printf("FAIL %s n=%d: left %d info %d\n", name, n, left, info);
+        ++failures;
+        return;
+    }
+    if (left) {
+        std::printf("pass %-22s n=%3d Hermitian, left to the FP64 kernels\n", name, n);
+        return;
+    }
+    for (int by = 0; by * 32 < n; ++by) {
+        blockIdx.y = by;
+        run_cta(32, (size_t)n * 32 * sizeof(lz), [&] { fix_apply_kernel(n, 1, Q.data(), nn, log.data(), (long long)log.size(), table.data(), head, &status); });
+        run_cta(32, (size_t)n * 32 * 8, [&] { herm_apply_real_kernel(n, 1, Y.data(), ws.data(), &info); });
+    }
+    blockIdx.y = 0;
+    M Yc(nn), h(nn);
+    for (long long k = 0; k < nn; ++k) Yc[k] = zc{Y[k], 0};
+    for (int j = 0; j < n; ++j)
+        for (int i = 0; i < n; ++i) {
+            const zc x = a[(size_t)j * n + i], y = a[(size_t)i * n + j];
+            h[(size_t)j * n + i] = zc{0.5 * (x.re + y.re), 0.5 * (x.im - y.im)};
+        }
+    const M V = product(n, Q, Yc), HV = product(n, h, V);
+    double fro = 0, orth = 0, worst = 0;
+    for (const zc& z : h) fro += norm2(z);
+    fro = std::sqrt(fro);
+    for (int j = 0; j < n; ++j) {
+        double r = 0;
+        for (int i = 0; i < n; ++i) r += norm2(HV[(size_t)j * n + i] - w[j].re * V[(size_t)j * n + i]);
+        worst = std::max(worst, std::sqrt(r) / fro);
+        for (int k = 0; k <= j; ++k) {
+            zc s{0, 0};
+            for (int i = 0; i < n; ++i) s = zmacc(V[(size_t)k * n + i], V[(size_t)j * n + i], s);
+            orth = std::max(orth, zabs(s - zc{j == k ? 1.0 : 0.0, 0}));
+        }
+    }
+    const bool ok = orth <= 1e-13 && worst <= 1e-13;
+    std::printf("%s %-22s n=%3d Hermitian: rotations %.2f n^2, orthogonality %.1e, eigenpairs %.1e\n", ok ? "pass" : "FAIL", name, n,
+                (double)rot / nn, orth, worst);
     failures += !ok;
 }
 
@@ -243,6 +300,20 @@ int main() {
         d[77].im = NAN;
         solve("not finite", 30, d, 4, 1);
         solve("tiny", 30, random(30, 1e-290), 4, 1);
+    }
+    for (int n : {2, 3, 17, 32, 33, 65, 97}) solve_hermitian("random", n, random(n, 1.0), 4, 0);
+    solve_hermitian("random, small scale", 40, random(40, 1e-30), 4, 0);
+    for (int n : {41, 121}) solve_hermitian("lossless grating", n, layer(n, 0.0), 4, 0);
+    {
+        M a((size_t)50 * 50, zc{0, 0}), w21((size_t)41 * 41, zc{0, 0});
+        for (int i = 0; i < 50; ++i) a[(size_t)i * 50 + i] = zc{(double)(i / 5) - 3, 0.0};
+        solve_hermitian("diagonal, repeated", 50, a, 4, 0);
+        for (int i = 0; i < 41; ++i) {  // Wilkinson's W+: pairs of eigenvalues equal to many digits
+            w21[(size_t)i * 41 + i] = zc{std::fabs(i - 20.0), 0};
+            if (i) w21[(size_t)i * 41 + i - 1] = w21[(size_t)(i - 1) * 41 + i] = zc{1, 0};
+        }
+        solve_hermitian("Wilkinson W+", 41, w21, 4, 0);
+        solve_hermitian("zero", 30, M((size_t)900, zc{0, 0}), 4, 1);
     }
     std::printf("%s\n", failures ? "FAILED" : "OK");
     return failures ? 1 : 0;

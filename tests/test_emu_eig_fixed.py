@@ -4,7 +4,9 @@ on 200,000 triples against long double (within 2^-57, a sixteenth of FP64's roun
 matrices of orders 2..97 (the edges of the 32-column blocks and tiles), matrices scaled by 1e-30 and 1e40,
 absorbing and lossless grating layers up to order 161, diagonal and triangular matrices with repeated entries,
 blocks of very different size, and what is left to the FP64 kernels (zero, non-finite and extreme matrices, one
-that needs an exceptional shift beyond the scale). Orthogonality, Schur residual and eigenpair residuals are held
+that needs an exceptional shift beyond the scale); and the Hermitian solver's pieces (the reduction, the QL
+iteration, both sets of rotations) on random Hermitian, lossless grating, diagonal and Wilkinson W+ matrices.
+Orthogonality, Schur residual and eigenpair residuals are held
 to 1e-13, the bound of the FP64 solver's tests."""
 import os
 import shutil
@@ -25,4 +27,4 @@ def test_fixed_point_eigensolver_in_emulation(tmp_path):
     assert build.returncode == 0, build.stderr[-2000:]
     run = subprocess.run([str(exe)], capture_output=True, text=True, timeout=900)
     assert run.returncode == 0 and run.stdout.strip().endswith("OK"), run.stdout[-3000:]
-    assert run.stdout.count("pass ") == 28
+    assert run.stdout.count("pass ") == 41

@@ -68,3 +68,20 @@ def test_matrices_left_to_the_fp64_kernels(eng):
     for k in (0, 2, 4, 5):
         r = np.linalg.norm(a[k] @ v[k] - v[k] * w[k], axis=0)
         assert r.max() <= 1e-13 * np.linalg.norm(a[k])
+
+
+@pytest.mark.parametrize("n,batch", [(24, 4), (32, 4), (33, 1400), (65, 3), (121, 396), (121, 397), (301, 2), (440, 1)])
+def test_hermitian(eng, n, batch):
+    """Both sides of the fixed-point reduction's limit (n * batch = 48000) and of its orders."""
+    rng = np.random.default_rng(n + batch)
+    few = np.stack([layer(n, rng) for _ in range(min(batch, 4))])
+    few = 0.5 * (few + few.conj().transpose(0, 2, 1))
+    a = few[np.arange(batch) % len(few)]
+    if batch > 4:
+        a[5] = 0.0  # left to the FP64 kernels
+    w, v, info = eng.eig_hermitian_batch(a)
+    assert (info == 0).all()
+    for k in range(min(batch, 7)):
+        r = np.linalg.norm(a[k] @ v[k] - v[k] * w[k], axis=0)
+        assert r.max() <= 1e-13 * np.linalg.norm(a[k])
+        assert np.abs(v[k].conj().T @ v[k] - np.eye(n)).max() <= 1e-13
