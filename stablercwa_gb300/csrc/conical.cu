@@ -1593,12 +1593,12 @@ void solve_conical_device(cudaStream_t st, const rcwa_stack1d& stack, const Coni
             mem.free(rhs);
             zc* t1 = mem.get<zc>(2 * nv);
             zc* t2 = mem.get<zc>(2 * nv);
-            LAUNCH(matvec_kernel, warp_blocks(B), 128, st, B, n, 2, r.p, down, down, t1, 1.0, 1.0);
-            LAUNCH(matvec_kernel, warp_blocks(B), 128, st, B, n, 2, r.p, down, down, t2, -1.0, 1.0);
+            LAUNCH(matvec_kernel, matvec_grid(B, n), kMatvecThreads, st, B, n, 2, r.p, down, down, t1, 1.0, 1.0);
+            LAUNCH(matvec_kernel, matvec_grid(B, n), kMatvecThreads, st, B, n, 2, r.p, down, down, t2, -1.0, 1.0);
             zc* X = mem.get<zc>(2 * nv);
             zc* Y = mem.get<zc>(2 * nv);
-            LAUNCH(matvec_kernel, warp_blocks(B), 128, st, B, n, 2, modes[1].W, t1, nullptr, X, 1.0, 0.0);
-            LAUNCH(matvec_kernel, warp_blocks(B), 128, st, B, n, 2, modes[1].V, t2, nullptr, Y, 1.0, 0.0);
+            LAUNCH(matvec_kernel, matvec_grid(B, n), kMatvecThreads, st, B, n, 2, modes[1].W, t1, nullptr, X, 1.0, 0.0);
+            LAUNCH(matvec_kernel, matvec_grid(B, n), kMatvecThreads, st, B, n, 2, modes[1].V, t2, nullptr, Y, 1.0, 0.0);
             LAUNCH(conical_top_reflection_kernel, nblocks(2 * nv), kTpb, st, B, n, N, M, modes[0].w, modes[0].v, X, Y, rud);
             for (zc* ptr : {t1, t2, X, Y}) mem.free(ptr);
         } else {
@@ -1623,8 +1623,8 @@ void solve_conical_device(cudaStream_t st, const rcwa_stack1d& stack, const Coni
                 LAUNCH(col_extract_kernel, nblocks(nv), kTpb, st, B, n, tm, N + M, tm_e, 2, 1);
                 LAUNCH(col_extract_kernel, nblocks(nv), kTpb, st, B, n, tp, M, tdd, 2, 0);
                 LAUNCH(col_extract_kernel, nblocks(nv), kTpb, st, B, n, tp, N + M, tdd, 2, 1);
-                LAUNCH(matvec_kernel, warp_blocks(B), 128, st, B, n, 2, rdu, tm_e, tdd, tdd, -1.0, 1.0);
-                LAUNCH(matvec_kernel, warp_blocks(B), 128, st, B, n, 2, tpi, tm_e, nullptr, rud, -1.0, 0.0);
+                LAUNCH(matvec_kernel, matvec_grid(B, n), kMatvecThreads, st, B, n, 2, rdu, tm_e, tdd, tdd, -1.0, 1.0);
+                LAUNCH(matvec_kernel, matvec_grid(B, n), kMatvecThreads, st, B, n, 2, tpi, tm_e, nullptr, rud, -1.0, 0.0);
                 mem.free(tp);
                 mem.free(tm);
                 topRdu = {KDense, rdu};
@@ -1639,9 +1639,9 @@ void solve_conical_device(cudaStream_t st, const rcwa_stack1d& stack, const Coni
                 down = solve(c, k.p, true, RHS_DENSE, tdd, 2);
             }
             zc* rdn = mem.get<zc>(2 * nv);
-            LAUNCH(apply_g_kernel, warp_blocks(B), 128, st, B, n, 2, (int)r.kind, r.p, nullptr, nullptr, down, rdn);
+            LAUNCH(apply_g_kernel, matvec_grid(B, n), kMatvecThreads, st, B, n, 2, (int)r.kind, r.p, nullptr, nullptr, down, rdn);
             zc* back = mem.get<zc>(2 * nv);
-            LAUNCH(apply_g_kernel, warp_blocks(B), 128, st, B, n, 2, (int)topTuu.kind, topTuu.p, nullptr, nullptr, rdn, back);
+            LAUNCH(apply_g_kernel, matvec_grid(B, n), kMatvecThreads, st, B, n, 2, (int)topTuu.kind, topTuu.p, nullptr, nullptr, rdn, back);
             LAUNCH(vec_add_kernel, nblocks(2 * nv), kTpb, st, 2 * nv, back, rud);
         }
         zc* cur = down;
@@ -1658,7 +1658,7 @@ void solve_conical_device(cudaStream_t st, const rcwa_stack1d& stack, const Coni
             if (g[b].kind == KSeam)
                 apply_seam(c, g[b], 2, cur, seam_t, nxt);
             else
-                LAUNCH(apply_g_kernel, warp_blocks(B), 128, st, B, n, 2, (int)g[b].kind, g[b].p, g[b].alt, g[b].alt_flag,
+                LAUNCH(apply_g_kernel, matvec_grid(B, n), kMatvecThreads, st, B, n, 2, (int)g[b].kind, g[b].p, g[b].alt, g[b].alt_flag,
                        cur, nxt);
             std::swap(cur, nxt);
             if (fields && b % 2 != 0) {  // the reflection below applied at the layer's bottom (:926-931)
@@ -1671,7 +1671,7 @@ void solve_conical_device(cudaStream_t st, const rcwa_stack1d& stack, const Coni
                     bottom = cleared;
                 }
                 cap.a_minus[j] = mem.get<zc>(2 * nv);
-                LAUNCH(apply_g_kernel, warp_blocks(B), 128, st, B, n, 2, (int)cap.r_below[j].kind, cap.r_below[j].p, nullptr,
+                LAUNCH(apply_g_kernel, matvec_grid(B, n), kMatvecThreads, st, B, n, 2, (int)cap.r_below[j].kind, cap.r_below[j].p, nullptr,
                        nullptr, bottom, cap.a_minus[j]);
                 if (pure_films)
                     LAUNCH(conical_clear_unexcited_kernel, nblocks(2 * nv), kTpb, st, 2 * nv, n, N, M, cap.a_minus[j]);

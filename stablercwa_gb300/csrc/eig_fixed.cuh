@@ -982,7 +982,7 @@ static __global__ void __launch_bounds__(128) fix_unit_columns_kernel(int n, int
 // herm_ql_kernel's iteration (eig.cuh: implicit QL with Wilkinson's shift on d and e, one thread per matrix, every
 // rotation logged for herm_apply_real_kernel) in fixed point. Its chain of about 20 dependent FP64 instructions a
 // rotation, 64 cycles each, took 1.1 us (17.2 ms for one matrix of order 121); the same chain in integers takes
-// 0.5 us (7.4 ms), and 4096 matrices' 20 ms went to MEASURED_Q. d and e are scaled so that
+// 0.5 us (7.4 ms), and 4096 matrices' 20 ms went to 8.3. d and e are scaled so that
 // N >= ||T||_2 (Gershgorin's bound) lies in [2^58, 2^59) units: the iteration's quantities stay below 4 N. What it does
 // not finish (non-finite or zero matrices, scales whose powers of two are not normal doubles, 30 sweeps without a
 // deflation) is flagged as a full log is, for the fused FP64 kernel. status, if given: matrices whose reduction left

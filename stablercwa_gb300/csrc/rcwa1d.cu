@@ -674,9 +674,9 @@ void solve1d_device(cudaStream_t st, const rcwa_stack1d& stack, const double* d_
             mem.free(P);
             mem.free(rhs);
             zc* t = c.vec();
-            LAUNCH(matvec_kernel, warp_blocks(B), 128, st, B, n, 1, r.p, down, down, t, 1.0, 1.0);
+            LAUNCH(matvec_kernel, matvec_grid(B, n), kMatvecThreads, st, B, n, 1, r.p, down, down, t, 1.0, 1.0);
             Rv = c.vec();
-            LAUNCH(matvec_kernel, warp_blocks(B), 128, st, B, n, 1, modes[1].W, t, nullptr, Rv, 1.0, 0.0);
+            LAUNCH(matvec_kernel, matvec_grid(B, n), kMatvecThreads, st, B, n, 1, modes[1].W, t, nullptr, Rv, 1.0, 0.0);
             LAUNCH(sub_incident_kernel, nblocks(B), kTpb, st, B, n, M, Rv);
             mem.free(t);
         } else {
@@ -700,8 +700,8 @@ void solve1d_device(cudaStream_t st, const rcwa_stack1d& stack, const double* d_
                 zc* tm_e = c.vec();
                 LAUNCH(col_extract_kernel, nblocks(nv), kTpb, st, B, n, tm, M, tm_e, 1, 0);
                 LAUNCH(col_extract_kernel, nblocks(nv), kTpb, st, B, n, tp, M, tdd, 1, 0);
-                LAUNCH(matvec_kernel, warp_blocks(B), 128, st, B, n, 1, rdu, tm_e, tdd, tdd, -1.0, 1.0);
-                LAUNCH(matvec_kernel, warp_blocks(B), 128, st, B, n, 1, tpi, tm_e, nullptr, rud, -1.0, 0.0);
+                LAUNCH(matvec_kernel, matvec_grid(B, n), kMatvecThreads, st, B, n, 1, rdu, tm_e, tdd, tdd, -1.0, 1.0);
+                LAUNCH(matvec_kernel, matvec_grid(B, n), kMatvecThreads, st, B, n, 1, tpi, tm_e, nullptr, rud, -1.0, 0.0);
                 mem.free(tp);
                 mem.free(tm);
                 topRdu = {KDense, rdu};
@@ -717,9 +717,9 @@ void solve1d_device(cudaStream_t st, const rcwa_stack1d& stack, const double* d_
             }
             // R = rud + Tuu (r down)
             zc* rdn = c.vec();
-            LAUNCH(apply_g_kernel, warp_blocks(B), 128, st, B, n, 1, (int)r.kind, r.p, nullptr, nullptr, down, rdn);
+            LAUNCH(apply_g_kernel, matvec_grid(B, n), kMatvecThreads, st, B, n, 1, (int)r.kind, r.p, nullptr, nullptr, down, rdn);
             zc* back = c.vec();
-            LAUNCH(apply_g_kernel, warp_blocks(B), 128, st, B, n, 1, (int)topTuu.kind, topTuu.p, nullptr, nullptr, rdn, back);
+            LAUNCH(apply_g_kernel, matvec_grid(B, n), kMatvecThreads, st, B, n, 1, (int)topTuu.kind, topTuu.p, nullptr, nullptr, rdn, back);
             LAUNCH(vec_add_kernel, nblocks(nv), kTpb, st, nv, back, rud);  // rud = back + rud
             Rv = rud;
         }
@@ -743,7 +743,7 @@ void solve1d_device(cudaStream_t st, const rcwa_stack1d& stack, const double* d_
             if (g[b].kind == KSeam) {
                 apply_seam(c, g[b], 1, cur, seam_t, nxt);
             } else {
-                LAUNCH(apply_g_kernel, warp_blocks(B), 128, st, B, n, 1, (int)g[b].kind, g[b].p, g[b].alt, g[b].alt_flag,
+                LAUNCH(apply_g_kernel, matvec_grid(B, n), kMatvecThreads, st, B, n, 1, (int)g[b].kind, g[b].p, g[b].alt, g[b].alt_flag,
                        cur, nxt);
             }
             std::swap(cur, nxt);
@@ -755,7 +755,7 @@ void solve1d_device(cudaStream_t st, const rcwa_stack1d& stack, const double* d_
                     LAUNCH(clear_unexcited_kernel, nblocks(nv), kTpb, st, B, n, M, bottom);
                 }
                 a_minus[j] = c.vec();
-                LAUNCH(apply_g_kernel, warp_blocks(B), 128, st, B, n, 1, (int)r_below[j].kind, r_below[j].p, nullptr, nullptr,
+                LAUNCH(apply_g_kernel, matvec_grid(B, n), kMatvecThreads, st, B, n, 1, (int)r_below[j].kind, r_below[j].p, nullptr, nullptr,
                        bottom, a_minus[j]);
                 if (pure_films) {
                     LAUNCH(clear_unexcited_kernel, nblocks(nv), kTpb, st, B, n, M, a_minus[j]);

@@ -790,7 +790,7 @@ void solve2d_host(cudaStream_t st, const rcwa_stack2d& stack, const rcwa_point2d
                     LAUNCH(bd_apply_vec_kernel, nblocks((long long)B * N), kTpb, st, B, N, tdd, inc, rhs);
                     down = solve(c, mat, true, RHS_DENSE, rhs, 1);
                     zc* back = c.vec();
-                    LAUNCH(matvec_kernel, warp_blocks(B), 128, st, B, n, 1, r.p, down, nullptr, back, 1.0, 0.0);
+                    LAUNCH(matvec_kernel, matvec_grid(B, n), kMatvecThreads, st, B, n, 1, r.p, down, nullptr, back, 1.0, 0.0);
                     LAUNCH(top_bd_finish_kernel, nblocks((long long)B * N), kTpb, st, B, N, rud, tuu, inc, back, R);
                     for (zc* p : {tdd, rdu, rud, tuu, mat, rhs, back}) mem.free(p);
                 }
@@ -813,7 +813,7 @@ void solve2d_host(cudaStream_t st, const rcwa_stack2d& stack, const rcwa_point2d
                 zc* rhs = c.vec();
                 LAUNCH(scale_vec_kernel, nblocks((long long)B * n), kTpb, st, (long long)B * n, inc, 2.0, rhs);
                 down = solve(c, kmat, true, RHS_DENSE, rhs, 1);
-                LAUNCH(matvec_kernel, warp_blocks(B), 128, st, B, n, 1, wp, down, inc, R, 1.0, -1.0);
+                LAUNCH(matvec_kernel, matvec_grid(B, n), kMatvecThreads, st, B, n, 1, wp, down, inc, R, 1.0, -1.0);
                 mem.free(kmat);
                 mem.free(rhs);
                 if (own) {
@@ -837,11 +837,11 @@ void solve2d_host(cudaStream_t st, const rcwa_stack2d& stack, const rcwa_point2d
                 LAUNCH(bd_apply_vec_kernel, nblocks((long long)B * N), kTpb, st, B, N, s.bd, down, y);
             } else {
                 zc* u = c.vec();
-                LAUNCH(matvec_kernel, warp_blocks(B), 128, st, B, n, 1, s.rp, down, down, u, 1.0, 1.0);  // (I + r') v
+                LAUNCH(matvec_kernel, matvec_grid(B, n), kMatvecThreads, st, B, n, 1, s.rp, down, down, u, 1.0, 1.0);  // (I + r') v
                 if (s.kind == S_IFACE_DENSE) {
                     zc* w = c.vec();
-                    LAUNCH(matvec_kernel, warp_blocks(B), 128, st, B, n, 1, s.nn, down, nullptr, w, 1.0, 0.0);
-                    LAUNCH(matvec_kernel, warp_blocks(B), 128, st, B, n, 1, s.tm, u, w, y, 1.0, 1.0);
+                    LAUNCH(matvec_kernel, matvec_grid(B, n), kMatvecThreads, st, B, n, 1, s.nn, down, nullptr, w, 1.0, 0.0);
+                    LAUNCH(matvec_kernel, matvec_grid(B, n), kMatvecThreads, st, B, n, 1, s.tm, u, w, y, 1.0, 1.0);
                     mem.free(w);
                 } else {
                     LAUNCH(iface_bd_step_kernel, nblocks((long long)B * N), kTpb, st, B, N, s.tm, s.nn, u, down, y);
@@ -861,7 +861,7 @@ void solve2d_host(cudaStream_t st, const rcwa_stack2d& stack, const rcwa_point2d
                 else if (rb.kind == R_BD)
                     LAUNCH(bd_apply_vec_kernel, nblocks((long long)B * N), kTpb, st, B, N, rb.p, down, am);
                 else
-                    LAUNCH(matvec_kernel, warp_blocks(B), 128, st, B, n, 1, rb.p, down, nullptr, am, 1.0, 0.0);
+                    LAUNCH(matvec_kernel, matvec_grid(B, n), kMatvecThreads, st, B, n, 1, rb.p, down, nullptr, am, 1.0, 0.0);
                 cap.a_minus[jl] = am;
             }
         }

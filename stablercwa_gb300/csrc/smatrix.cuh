@@ -55,49 +55,54 @@ __global__ void col_extract_kernel(int B, int n, const zc* __restrict__ m, int c
 
 // y = s_c * y0 + s_ab * (A x), warp per sample, lanes along rows; the sum over columns is ascending
 // like the reference's matrix-vector product (include/stablercwa/matrix.hpp:186-194).
-__global__ void matvec_kernel(int B, int n, int cols, const zc* __restrict__ A, const zc* __restrict__ x,
-                              const zc* y0, zc* y, double s_ab, double s_c) {
-    const long long b = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (b >= B) return;
-    const int lane = threadIdx.x & 31;
-    const zc* As = A + b * n * n;
+// A CTA per sample and 32 rows: a lane per row, the columns of A dealt to its four warps, their sums added in order
+// through shared memory. (A warp per sample took 1.0 ms for one matrix of order 338 on one SM.)
+constexpr int kMatvecThreads = 128;
+inline dim3 matvec_grid(int B, int n) { return dim3((unsigned)B, (unsigned)((n + 31) / 32)); }
+__device__ __forceinline__ zc matvec_row(int n, int i, const zc* __restrict__ As, const zc* __restrict__ xs) {
+    __shared__ zc part[4][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    zc acc = zc{0.0, 0.0};
+    if (i < n) {
+#pragma unroll 4
+        for (int k = warp; k < n; k += 4) acc = zmac(As[(long long)k * n + i], xs[k], acc);
+    }
+    part[warp][lane] = acc;
+    __syncthreads();
+    acc = (part[0][lane] + part[1][lane]) + (part[2][lane] + part[3][lane]);
+    __syncthreads();
+    return acc;
+}
+__global__ void __launch_bounds__(kMatvecThreads) matvec_kernel(int B, int n, int cols, const zc* __restrict__ A,
+                                                                const zc* __restrict__ x, const zc* y0, zc* y, double s_ab,
+                                                                double s_c) {
+    const long long b = blockIdx.x;
+    const int i = blockIdx.y * 32 + (threadIdx.x & 31);
     for (int c = 0; c < cols; ++c) {
         const long long base = (b * cols + c) * n;
-        const zc* xs = x + base;
-        for (int i = lane; i < n; i += 32) {
-            zc acc = zc{0.0, 0.0};
-            for (int k = 0; k < n; ++k) acc = zfma(As[(long long)k * n + i], xs[k], acc);
-            zc v = zc{s_ab * acc.re, s_ab * acc.im};
-            if (y0 && s_c != 0.0) v = zc{s_c * y0[base + i].re + v.re, s_c * y0[base + i].im + v.im};
-            y[base + i] = v;
-        }
+        const zc acc = matvec_row(n, i, A + b * n * n, x + base);
+        if (threadIdx.x >= 32 || i >= n) continue;
+        zc v = zc{s_ab * acc.re, s_ab * acc.im};
+        if (y0 && s_c != 0.0) v = zc{s_c * y0[base + i].re + v.re, s_c * y0[base + i].im + v.im};
+        y[base + i] = v;
     }
 }
 
-// g applied to a vector: diagonal g, or the per-sample dense alternative where alt_flag is set.
-__global__ void apply_g_kernel(int B, int n, int cols, int kind, const zc* __restrict__ g, const zc* __restrict__ alt,
-                               const int* __restrict__ alt_flag, const zc* __restrict__ x, zc* __restrict__ y) {
-    const long long b = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (b >= B) return;
-    const int lane = threadIdx.x & 31;
-    const bool dense = kind == 2 || (alt_flag && alt_flag[b]);
+// g applied to a vector: diagonal g, or the per-sample dense alternative where alt_flag is set; matvec_kernel's grid.
+__global__ void __launch_bounds__(kMatvecThreads) apply_g_kernel(int B, int n, int cols, int kind, const zc* __restrict__ g,
+                                                                 const zc* __restrict__ alt, const int* __restrict__ alt_flag,
+                                                                 const zc* __restrict__ x, zc* __restrict__ y) {
+    const long long b = blockIdx.x;
+    const int i = blockIdx.y * 32 + (threadIdx.x & 31);
+    const bool dense = kind == 2 || (kind != 0 && alt_flag && alt_flag[b]);
     const zc* Ms = kind == 2 ? g + b * n * n : (alt ? alt + b * n * n : nullptr);
     for (int c = 0; c < cols; ++c) {
         const long long base = (b * cols + c) * n;
-        const zc* xs = x + base;
-        for (int i = lane; i < n; i += 32) {
-            zc v;
-            if (kind == 0) {
-                v = zc{0.0, 0.0};
-            } else if (!dense) {
-                v = g[b * n + i] * xs[i];
-            } else {
-                zc acc = zc{0.0, 0.0};
-                for (int k = 0; k < n; ++k) acc = zfma(Ms[(long long)k * n + i], xs[k], acc);
-                v = acc;
-            }
-            y[base + i] = v;
-        }
+        zc v = zc{0.0, 0.0};
+        if (dense) v = matvec_row(n, i, Ms, x + base);
+        if (threadIdx.x >= 32 || i >= n) continue;
+        if (!dense && kind != 0) v = g[b * n + i] * x[base + i];
+        y[base + i] = v;
     }
 }
 
@@ -359,9 +364,9 @@ Seam analytic_over_dense_seam(Batch& c, const zc* W, const zc* V, const zc* w, c
 
 // y = g x for a KSeam g = tp + tm r' (cols right-hand sides); t is scratch of the size of x
 inline void apply_seam(Batch& c, const DOp& g, int cols, const zc* x, zc* t, zc* y) {
-    LAUNCH(matvec_kernel, warp_blocks(c.B), 128, c.st, c.B, c.n, cols, g.rp, x, nullptr, t, 1.0, 0.0);
-    LAUNCH(matvec_kernel, warp_blocks(c.B), 128, c.st, c.B, c.n, cols, g.alt, t, nullptr, y, 1.0, 0.0);
-    LAUNCH(matvec_kernel, warp_blocks(c.B), 128, c.st, c.B, c.n, cols, g.p, x, y, y, 1.0, 1.0);
+    LAUNCH(matvec_kernel, matvec_grid(c.B, c.n), kMatvecThreads, c.st, c.B, c.n, cols, g.rp, x, nullptr, t, 1.0, 0.0);
+    LAUNCH(matvec_kernel, matvec_grid(c.B, c.n), kMatvecThreads, c.st, c.B, c.n, cols, g.alt, t, nullptr, y, 1.0, 0.0);
+    LAUNCH(matvec_kernel, matvec_grid(c.B, c.n), kMatvecThreads, c.st, c.B, c.n, cols, g.p, x, y, y, 1.0, 1.0);
 }
 
 // ---------------------------------------------------------------- Fourier coefficients (host)
