@@ -190,12 +190,13 @@ void herm_panel_launch(cudaStream_t st, int n, int batch, int k0, const zc* a, l
 // trailing block's rank-2 nb update A -= V W^H + W V^H as two batched products (the tensor cores for
 // orders >= 32). vall receives the reflectors, mall the panels' T V^H.
 void herm_blocked_reduce(cudaStream_t st, int n, int batch, const zc* a, long long a_stride, zc* ws, zc* pan, zc* vall,
-                         zc* mall, int group) {
+                         zc* mall, int group, bool fixed) {
     const int nb = kHermNb, P = herm_panel_count(n), pnb = P * nb;
     const long long ws_stride = eig_workspace_elems(n), pan_stride = herm_panel_elems(n);
     for (int b = 0; b < P; ++b) {
         const int k0 = b * nb;
-        switch (group) {
+        if (fixed) launch_herm_panel_fixed(st, n, batch, k0, a, a_stride, ws, pan, vall, mall, pnb, group);
+        else switch (group) {
             case 4: herm_panel_launch<4>(st, n, batch, k0, a, a_stride, ws, pan, vall, mall, pnb); break;
             case 8: herm_panel_launch<8>(st, n, batch, k0, a, a_stride, ws, pan, vall, mall, pnb); break;
             case 16: herm_panel_launch<16>(st, n, batch, k0, a, a_stride, ws, pan, vall, mall, pnb); break;
@@ -260,12 +261,14 @@ bool herm_blocked_wanted(int n, int group) {
     return group <= 32 && n >= 64 && tc_gemm_enabled() && !Fp64ProductsGuard::active();
 }
 
-// The fixed-point reduction (a CTA per matrix) against the FP64 ones (lane groups, blocked from order 64; a CTA for
-// few matrices), whole eigensolves in ms: order 121: 1 matrix 14.2 / 20.2, 304 23.2 / 28.6, 608 35.4 / 34.2, 4096
-// 170 / 127; order 301: 1 88 / 193, 152 225 / 283, 304 390 / 289; order 161: 304 54 / 59, 1000 137 / 94; order 61:
-// 1 4.2 / 5.8, 1000 10.1 / 11.0; order 41: 1 2.0 / 2.7, 4000 12.5 / 10.5. The line lies where n * batch matrices'
-// columns fill the GPU's SMs about three deep.
-bool herm_fixed_reduce_wanted(int n, int batch) { return (long long)n * batch <= 48000 && eig_fixed_possible(n); }
+// The fixed-point reduction by rotations (a CTA per matrix) against the lane groups' Householder reduction (FP64; blocked
+// from order 64, there with fixed-point panels), whole eigensolves in ms: order 41: 1 matrix 2.0 / 2.7, 4000 12.5 / 10.5;
+// order 61: 1 4.2 / 5.8, 1000 10.1 / 11.0; order 81: 304 9.8 / 10.6, 592 14.1 / 12.7; order 121: 64 17.2 / 23.2, 304
+// 23.4 / 25.0, 396 30.1 / 27.6; order 161: 298 54 / 68; order 301: 16 115 / 213, 159 275 / 308. The line lies where
+// n * batch matrices' columns fill the GPU's SMs about three deep, for the blocked form at most 360 matrices.
+bool herm_fixed_reduce_wanted(int n, int batch) {
+    return (long long)n * batch <= 48000 && (n < 64 || batch <= 360) && eig_fixed_possible(n);
+}
 
 void herm_fused_dispatch(cudaStream_t st, int n, int batch, const zc* a, long long a_stride, zc* w, zc* v, int* info,
                          zc* ws, double eps, int max_iter, int group, const int* only) {
@@ -315,7 +318,7 @@ void launch_eig_herm(cudaStream_t st, int n, int batch, const zc* a, long long a
         RCWA_CUDA(cudaMallocAsync(&pan, (size_t)batch * herm_panel_elems(n) * sizeof(zc), st));
         RCWA_CUDA(cudaMallocAsync(&mall, (size_t)batch * pnb * n * sizeof(zc), st));
         RCWA_CUDA(cudaMallocAsync(&u, (size_t)batch * kHermNb * n * sizeof(zc), st));
-        herm_blocked_reduce(st, n, batch, a, a_stride, ws, pan, q, mall, group);
+        herm_blocked_reduce(st, n, batch, a, a_stride, ws, pan, q, mall, group, fixed);
     } else if (fixed_reduce) {
         RCWA_CUDA(cudaMallocAsync(&status, (size_t)batch * sizeof(int), st));
         launch_herm_reduce_fixed(st, n, batch, a, a_stride, q, ws, status);

@@ -861,6 +861,31 @@ constexpr int kHermNb = 32;
 __host__ __device__ inline long long herm_panel_elems(int n) { return 4LL * kHermNb * n + kHermNb * kHermNb + kHermNb; }
 __host__ __device__ inline int herm_panel_count(int n) { return n > 1 ? (n - 2) / kHermNb + 1 : 0; }
 
+// the trailing update's second operand, and M = T V^H (rows of V above k0 + 1 are zero)
+template <int G>
+__device__ __forceinline__ void herm_panel_finish(int n, int k0, int nbp, const zc* __restrict__ VW, zc* __restrict__ Bt,
+                                                  const zc* __restrict__ T, zc* __restrict__ mall, int pnb) {
+    constexpr int nb = kHermNb;
+    const int g = threadIdx.x & (G - 1);
+    const zc zero{0.0, 0.0};
+    for (int r = g; r < n; r += G) {
+        zc* bt = Bt + (long long)r * 2 * nb;
+        for (int q = 0; q < nb; ++q) {
+            bt[q] = conj(VW[(long long)(nb + q) * n + r]);
+            bt[nb + q] = conj(VW[(long long)q * n + r]);
+        }
+    }
+    const int b = k0 / nb;
+    for (int r = first_owned<G>(k0 + 1, g); r < n; r += G) {
+        zc* m = mall + (long long)r * pnb + b * nb;
+        for (int p = 0; p < nbp; ++p) {
+            zc acc = zero;
+            for (int q = p; q < nbp; ++q) acc = zmac(T[q * nb + p], conj(VW[(long long)q * n + r]), acc);
+            m[p] = acc;
+        }
+    }
+}
+
 template <int G>
 __device__ void herm_panel_one(int n, int k0, const zc* __restrict__ A0, zc* __restrict__ ws, zc* __restrict__ pan,
                                zc* __restrict__ vall, zc* __restrict__ mall, int pnb) {
@@ -1000,23 +1025,7 @@ __device__ void herm_panel_one(int n, int k0, const zc* __restrict__ A0, zc* __r
         d[n - 1] = a.re;
         e[n - 1] = 0.0;
     }
-    // the trailing update's second operand, and M = T V^H (rows of V above k0 + 1 are zero)
-    for (int r = g; r < n; r += G) {
-        zc* bt = Bt + (long long)r * 2 * nb;
-        for (int q = 0; q < nb; ++q) {
-            bt[q] = conj(VW[(long long)(nb + q) * n + r]);
-            bt[nb + q] = conj(VW[(long long)q * n + r]);
-        }
-    }
-    const int b = k0 / nb;
-    for (int r = first_owned<G>(k0 + 1, g); r < n; r += G) {
-        zc* m = mall + (long long)r * pnb + b * nb;
-        for (int p = 0; p < nbp; ++p) {
-            zc acc = zero;
-            for (int q = p; q < nbp; ++q) acc = zmac(T[q * nb + p], conj(VW[(long long)q * n + r]), acc);
-            m[p] = acc;
-        }
-    }
+    herm_panel_finish<G>(n, k0, nbp, VW, Bt, T, mall, pnb);
 }
 
 template <int G>

@@ -2,7 +2,7 @@
 #include <algorithm>
 #include <cstdlib>
 
-#include "eig_fixed.cuh"
+#include "herm_fixed.cuh"
 #include "engine.h"
 
 namespace rcwa_gb300 {
@@ -118,6 +118,28 @@ void launch_herm_ql_fixed(cudaStream_t st, int n, int batch, zc* w, int* info, z
     if (smem > 48 * 1024) ensure_smem_optin(reinterpret_cast<const void*>(herm_ql_fixed_kernel), (int)smem);
     herm_ql_fixed_kernel<<<(unsigned)((batch + kHermQlThreads - 1) / kHermQlThreads), kHermQlThreads, smem, st>>>(
         n, batch, w, info, ws, status, rotation_counter());
+    RCWA_CUDA(cudaGetLastError());
+}
+
+namespace {
+template <int G>
+void panel_launch(cudaStream_t st, int n, int batch, int k0, const zc* a, long long a_stride, zc* ws, zc* pan, zc* vall, zc* mall,
+                  int pnb) {
+    const unsigned blocks = (unsigned)(((long long)batch * G + 127) / 128);
+    herm_panel_fixed_kernel<G><<<blocks, 128, 0, st>>>(n, batch, k0, a, a_stride, ws, pan, vall, mall, pnb);
+}
+}  // namespace
+
+void launch_herm_panel_fixed(cudaStream_t st, int n, int batch, int k0, const zc* a, long long a_stride, zc* ws, zc* pan, zc* vall,
+                             zc* mall, int pnb, int group) {
+    switch (group) {
+        case 4: panel_launch<4>(st, n, batch, k0, a, a_stride, ws, pan, vall, mall, pnb); break;
+        case 8: panel_launch<8>(st, n, batch, k0, a, a_stride, ws, pan, vall, mall, pnb); break;
+        case 16: panel_launch<16>(st, n, batch, k0, a, a_stride, ws, pan, vall, mall, pnb); break;
+        case 32: panel_launch<32>(st, n, batch, k0, a, a_stride, ws, pan, vall, mall, pnb); break;
+        default: throw EngineError{RCWA_EINVAL, "eig: the blocked Hermitian reduction takes 4, 8, 16 or 32 lanes"};
+    }
+    ++launch_count();
     RCWA_CUDA(cudaGetLastError());
 }
 
