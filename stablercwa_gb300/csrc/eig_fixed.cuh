@@ -130,11 +130,13 @@ __device__ __forceinline__ int fix_tops(long long x, long long y, long long z) {
 // scaled so that the largest magnitude is in [2^60, 2^61).
 __device__ __forceinline__ FixRot fix_rotation_scaled(long long xr, long long xi, long long sub) {
     const FixLimb a = fix_split(xr), b = fix_split(xi), c = fix_split(sub);
-    // Q = (a^2 + b^2 + c^2) 2^-60, in [2^60, 3 2^62) (unsigned); + 1: the dropped squares of the low limbs on average
-    long long u = fix_mad(a.h, a.l, 1LL << 28);
+    // Q = (a^2 + b^2 + c^2) 2^-60, in [2^60, 3 2^62) (unsigned)
+    const unsigned long long ll = (unsigned long long)((unsigned)a.l) * (unsigned)a.l + (unsigned long long)((unsigned)b.l) * (unsigned)b.l +
+                                  (unsigned long long)((unsigned)c.l) * (unsigned)c.l;
+    long long u = fix_mad(a.h, a.l, (1LL << 28) + (long long)(ll >> 31));
     u = fix_mad(b.h, b.l, u);
     u = fix_mad(c.h, c.l, u);
-    long long Q = fix_mad(a.h, a.h, 1);
+    long long Q = fix_mad(a.h, a.h, 0);
     Q = fix_mad(b.h, b.h, Q);
     Q = fix_mad(c.h, c.h, Q);
     Q += u >> 29;
@@ -151,8 +153,10 @@ __device__ __forceinline__ FixRot fix_rotation_scaled(long long xr, long long xi
     const long long y = ((long long)y0 << 30) + (fix_mad((int)y0, d1, (fix_mad((int)y0, d0, 0) >> 21) + (1 << 10)) >> 11);  // 59 fractional bits
     const FixLimb Y = fix_split(y);
     const auto scale = [&](const FixLimb& x) {  // x y: 60 fractional bits
+        // (with the product of the low limbs: without its mean q and s came out a quarter of a unit low, |q|^2 + s^2
+        // below one, and the QL iteration, whose diagonal takes that as an addition, moved every small eigenvalue up)
         long long v = fix_mad(x.h, Y.l, (long long)(1 << 29));
-        v = fix_mad(x.l, Y.h, v);
+        v = fix_mad(x.l, Y.h, v) + (fix_mad(x.l, Y.l, 0) >> 30);
         return fix_mad(x.h, Y.h, v >> 30);
     };
     FixRot r;
@@ -982,12 +986,52 @@ static __global__ void __launch_bounds__(128) fix_unit_columns_kernel(int n, int
 // herm_ql_kernel's iteration (eig.cuh: implicit QL with Wilkinson's shift on d and e, one thread per matrix, every
 // rotation logged for herm_apply_real_kernel) in fixed point. Its chain of about 20 dependent FP64 instructions a
 // rotation, 64 cycles each, took 1.1 us (17.2 ms for one matrix of order 121); the same chain in integers takes
-// 0.5 us (7.4 ms), and 4096 matrices' 20 ms went to 8.3. d and e are scaled so that
-// N >= ||T||_2 (Gershgorin's bound) lies in [2^58, 2^59) units: the iteration's quantities stay below 4 N. What it does
+// 0.6 us (9.2 ms), and 4096 matrices' 20 ms went to 10. d and e are scaled so that
+// N >= ||T||_2 (Gershgorin's bound) lies in [2^58, 2^59) units: the iteration's quantities stay below 4 N. In memory d
+// and e have three more bits (|d|, |e| <= N fit), in the chain thirty (FixWide): with whole units throughout (7.4 ms),
+// the eigenvalues that are small beside N, a grating layer's propagating modes, came out up to three times as far off
+// as FP64's, whose rounding follows the entries; now they are closer (reflection amplitudes of order-301 layers, mean
+// relative error: FP64 5.4e-12, whole units 1.4e-11, these 2.2e-12). What it does
 // not finish (non-finite or zero matrices, scales whose powers of two are not normal doubles, 30 sweeps without a
 // deflation) is flagged as a full log is, for the fused FP64 kernel. status, if given: matrices whose reduction left
 // them to that kernel already.
 constexpr int kFixQlBits = 59;
+constexpr int kFixQlExtra = 3;  // bits below one unit of d and e in memory
+
+struct FixWide {  // y + x 2^-30 units, x in [0, 2^30)
+    long long y;
+    int x;
+};
+__device__ __forceinline__ FixWide fix_wide_unpack(long long v) {
+    return FixWide{v >> kFixQlExtra, (int)((unsigned)v & ((1u << kFixQlExtra) - 1)) << (30 - kFixQlExtra)};
+}
+__device__ __forceinline__ long long fix_wide_pack(const FixWide& a) {
+    return a.y * (1 << kFixQlExtra) + ((a.x + (1 << (29 - kFixQlExtra))) >> (30 - kFixQlExtra));
+}
+__device__ __forceinline__ FixWide fix_wide_add(const FixWide& a, const FixWide& b) {
+    const int x = a.x + b.x;
+    return FixWide{a.y + b.y + (x >> 30), x & 0x3fffffff};
+}
+__device__ __forceinline__ FixWide fix_wide_sub(const FixWide& a, const FixWide& b) {
+    const int x = a.x - b.x;
+    return FixWide{a.y - b.y + (x >> 30), x & 0x3fffffff};
+}
+// a b with the coefficient a = (a1, a0)
+__device__ __forceinline__ FixWide fix_wide_mul(int a1, int a0, const FixWide& b) {
+    const FixLimb l = fix_split(b.y);
+    const long long u2 = fix_mad(a0, l.l, fix_mad(a1, b.x, 1LL << 29));
+    const long long u = fix_mad(a0, l.h, fix_mad(a1, l.l, u2 >> 30));
+    return FixWide{fix_mad(a1, l.h, u >> 30), (int)((unsigned)u & 0x3fffffffu)};
+}
+// a b + c d; d's terms last
+__device__ __forceinline__ FixWide fix_wide_dot(int a1, int a0, const FixWide& b, int c1, int c0, const FixWide& d) {
+    const FixLimb l = fix_split(b.y), m = fix_split(d.y);
+    long long u2 = fix_mad(a0, l.l, fix_mad(a1, b.x, 1LL << 29));
+    long long u = fix_mad(a0, l.h, fix_mad(a1, l.l, 0));
+    u2 = fix_mad(c0, m.l, fix_mad(c1, d.x, u2));
+    u = fix_mad(c0, m.h, fix_mad(c1, m.l, u)) + (u2 >> 30);
+    return FixWide{fix_mad(c1, m.h, fix_mad(a1, l.h, 0)) + (u >> 30), (int)((unsigned)u & 0x3fffffffu)};
+}
 static __global__ void __launch_bounds__(kHermQlThreads) herm_ql_fixed_kernel(int n, int batch, zc* __restrict__ w,
                                                                              int* __restrict__ info, zc* __restrict__ ws,
                                                                              const int* __restrict__ status,
@@ -1025,8 +1069,8 @@ static __global__ void __launch_bounds__(kHermQlThreads) herm_ql_fixed_kernel(in
     info[gid] = 0;
     if (!usable) return;
     for (int k = 0; k < n; ++k) {
-        d[k * sd] = fix_from_double(src[k], e2);
-        e[k * sd] = k + 1 < n ? fix_from_double(src[n + k], e2) : 0;
+        d[k * sd] = fix_from_double(src[k], e2 - kFixQlExtra);
+        e[k * sd] = k + 1 < n ? fix_from_double(src[n + k], e2 - kFixQlExtra) : 0;
     }
     int2* table = reinterpret_cast<int2*>(reinterpret_cast<double*>(base) + 2 * n);
     int4* log = reinterpret_cast<int4*>(base + (long long)n * n);
@@ -1035,13 +1079,13 @@ static __global__ void __launch_bounds__(kHermQlThreads) herm_ql_fixed_kernel(in
     bool left = false;
     for (int l = 0; l < n && !left; ++l) {
         for (int its = 0;; ++its) {
-            // first m >= l with e[m] below eps (|d[m]| + |d[m+1]|), or of two units (2^-57 N at most)
+            // first m >= l with e[m] below eps (|d[m]| + |d[m+1]|), or of half a unit (2^-59 N at most)
             int m = l;
             for (; m < n - 1; ++m) {
                 const long long a = d[m * sd], b = d[(m + 1) * sd], x = e[m * sd];
                 const unsigned long long size = (unsigned long long)((a < 0 ? -a : a) + (b < 0 ? -b : b));
                 const unsigned long long ax = (unsigned long long)(x < 0 ? -x : x);
-                if (ax <= 2 || ax <= size >> 52) break;
+                if (ax <= 4 || ax <= size >> 52) break;
             }
             if (m == l) break;
             if (its == 30 || pos + (m - l) > log_cap || sweeps + 1 > table_cap) {
@@ -1050,58 +1094,60 @@ static __global__ void __launch_bounds__(kHermQlThreads) herm_ql_fixed_kernel(in
             }
             // g = d[m] - shift, the shift d[l] - e^2 / (h + sign(h) sqrt(h^2 + e^2)), h = (d[l+1] - d[l]) / 2, its
             // correction in float
-            long long g = d[m * sd] - d[l * sd];
+            FixWide g = fix_wide_sub(fix_wide_unpack(d[m * sd]), fix_wide_unpack(d[l * sd]));
             {
-                const float k = 0x1p-59f;
-                const float h = (float)((d[(l + 1) * sd] - d[l * sd]) >> 1) * k, x = (float)e[l * sd] * k;
+                const float k = 0x1p-62f;  // 2^-59 units
+                const float h = (float)((d[(l + 1) * sd] >> 1) - (d[l * sd] >> 1)) * k, x = (float)e[l * sd] * k;
                 const float den = h + copysignf(sqrtf(h * h + x * x), h);
-                if (fabsf(den) > 1e-18f) g += (long long)(x * (x / den) * 0x1p59f);
+                if (fabsf(den) > 1e-18f) g.y += (long long)(x * (x / den) * 0x1p59f);
             }
             FixRot q;  // c and s of the last rotation (c in q.cr, s in q.s)
             q.cr1 = q.s1 = 1 << 30;
             q.cr0 = q.s0 = 0;
-            long long p = 0;
+            FixWide p{0, 0};
             bool split = false;
             int i = m - 1;
-            long long ei = e[i * sd], di = d[i * sd], dn = d[m * sd];
+            FixWide ei = fix_wide_unpack(e[i * sd]), di = fix_wide_unpack(d[i * sd]), dn = fix_wide_unpack(d[m * sd]);
             for (; i >= l; --i) {
-                const FixLimb el = fix_split(ei), o{0, 0};
-                const long long b = fix_dot3(0, 0, o, 0, 0, o, q.cr1, q.cr0, el);
-                // f = s e exactly, 60 fractional bits in fl: where f and g are both small the angle between them,
-                // which carries the shift up the matrix, needs f's digits below one unit
-                const long long ll = fix_mad(q.s0, el.l, 0), u = fix_mad(q.s0, el.h, fix_mad(q.s1, el.l, ll >> 30));
-                const long long f = fix_mad(q.s1, el.h, u >> 30);
-                const unsigned long long fl = (unsigned long long)((unsigned)u & 0x3fffffffu) << 30 | ((unsigned)ll & 0x3fffffffu);
+                const FixLimb el = fix_split(ei.y);
+                const FixWide b = fix_wide_mul(q.cr1, q.cr0, ei);
+                // f = s e to the last digit, 60 fractional bits in fl: where f and g are both small the angle between
+                // them, which carries the shift up the matrix, needs f's digits below one unit
+                const long long ll = fix_mad(q.s0, el.l, fix_mad(q.s1, ei.x, fix_mad(q.s0, ei.x, 0) >> 30)),
+                                u = fix_mad(q.s0, el.h, fix_mad(q.s1, el.l, ll >> 30));
+                const FixWide f{fix_mad(q.s1, el.h, u >> 30), (int)((unsigned)u & 0x3fffffffu)};
+                const unsigned long long fl = (unsigned long long)f.x << 30 | ((unsigned)ll & 0x3fffffffu);
                 // the next rotation's entries, ahead of their use
                 const int in = i > l ? i - 1 : l;
                 const long long en = e[in * sd], dp = d[in * sd];
-                if (f == 0 && fl == 0 && g == 0) {
+                if (f.y == 0 && fl == 0 && g.y == 0 && g.x == 0) {
                     e[(i + 1) * sd] = 0;
-                    d[(i + 1) * sd] = dn - p;
+                    d[(i + 1) * sd] = fix_wide_pack(fix_wide_sub(dn, p));
                     e[m * sd] = 0;
                     split = true;
                     break;
                 }
                 {
-                    long long x = g, y = f;
-                    unsigned long long r = fl;
+                    long long x = g.y, y = f.y;
+                    unsigned long long r = fl, rx = (unsigned long long)g.x << 30;
                     int h = fix_tops(x, y, 0);
                     while (h == 0) {
-                        x <<= 28;
-                        y = y << 28 | (long long)(r >> 32);
+                        x = (long long)((unsigned long long)x << 28 | rx >> 32);
+                        rx = (rx << 28) & 0xfffffffffffffffull;
+                        y = (long long)((unsigned long long)y << 28 | r >> 32);
                         r = (r << 28) & 0xfffffffffffffffull;
                         h = fix_tops(x, y, 0);
                     }
                     const int sh = __clz(h) - 3;
-                    q = fix_rotation_scaled(x << sh, 0, y << sh | (long long)(r >> (60 - sh)));
+                    q = fix_rotation_scaled((long long)((unsigned long long)x << sh | rx >> (60 - sh)), 0,
+                                            (long long)((unsigned long long)y << sh | r >> (60 - sh)));
                 }
-                e[(i + 1) * sd] = fix_dot3(0, 0, o, q.s1, q.s0, fix_split(f), q.cr1, q.cr0, fix_split(g));
-                const long long g2 = dn - p;
-                const long long t = fix_dot3(0, 0, o, q.cr1, q.cr0, fix_split(2 * b), q.s1, q.s0, fix_split(di - g2));
-                const FixLimb tl = fix_split(t);
-                p = fix_dot3(0, 0, o, 0, 0, o, q.s1, q.s0, tl);
-                d[(i + 1) * sd] = g2 + p;
-                g = fix_dot3(0, 0, o, 0, 0, o, q.cr1, q.cr0, tl) - b;
+                e[(i + 1) * sd] = fix_wide_pack(fix_wide_dot(q.s1, q.s0, f, q.cr1, q.cr0, g));
+                const FixWide g2 = fix_wide_sub(dn, p);
+                const FixWide t = fix_wide_dot(q.cr1, q.cr0, fix_wide_add(b, b), q.s1, q.s0, fix_wide_sub(di, g2));
+                p = fix_wide_mul(q.s1, q.s0, t);
+                d[(i + 1) * sd] = fix_wide_pack(fix_wide_add(g2, p));
+                g = fix_wide_sub(fix_wide_mul(q.cr1, q.cr0, t), b);
                 // the log's form (herm_fixed_entry): s 2^62 and -c 2^62 in 31-bit limbs, saturated below 2^62
                 const long long s62 = min((((long long)q.s1 << 30) + q.s0) << 2, 0x3fffffffffffffffLL),
                                 c62 = min((((long long)q.cr1 << 30) + q.cr0) << 2, 0x3fffffffffffffffLL);
@@ -1109,13 +1155,13 @@ static __global__ void __launch_bounds__(kHermQlThreads) herm_ql_fixed_kernel(in
                 log[pos] = make_int4((int)(S >> 31), (int)(S & 0x7fffffff), (int)(C >> 31), (int)(C & 0x7fffffff));
                 ++pos;
                 dn = di;
-                ei = en;
-                di = dp;
+                ei = fix_wide_unpack(en);
+                di = fix_wide_unpack(dp);
             }
             const int first = split ? i + 1 : l;
             if (!split) {
-                d[l * sd] = dn - p;
-                e[l * sd] = g;
+                d[l * sd] = fix_wide_pack(fix_wide_sub(dn, p));
+                e[l * sd] = fix_wide_pack(g);
                 e[m * sd] = 0;
             }
             if (m - 1 >= first) table[sweeps++] = make_int2(first, m - 1);
@@ -1124,7 +1170,7 @@ static __global__ void __launch_bounds__(kHermQlThreads) herm_ql_fixed_kernel(in
     tail[0] = (int)sweeps;
     tail[1] = left;
     if (!left) {
-        const double unit = __longlong_as_double((long long)(e2 + 1023) << 52);
+        const double unit = __longlong_as_double((long long)(e2 - kFixQlExtra + 1023) << 52);
         for (int k = 0; k < n; ++k) w[gid * n + k] = zc{(double)d[k * sd] * unit, 0.0};
         if (rotations) atomicAdd(rotations, (unsigned long long)pos);
     }
