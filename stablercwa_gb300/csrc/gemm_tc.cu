@@ -21,12 +21,19 @@
 // Kernels. The split kernels write the digit planes in HBM as bf16 rows with K contiguous (K-major for
 // both operands), the second half of a complex K starting at Kp / 2. The product kernel gives each CTA one
 // 128 x 128 tile of C^ of one matrix: one warp issues TMA loads (128-byte swizzle, boxes of 128 rows x 64 K, two
-// of each operand a stage) into a 3-stage shared-memory ring; one thread issues tcgen05.mma (M = 128, N = 128,
-// K = 16, bf16 in, FP32 out) into one of two 128-column tensor-memory accumulators; eight warps read each finished
-// group out of tensor memory (tcgen05.ld) and add it, as an integer at its diagonal's weight, into one int64 per
-// element while the next group accumulates in the other buffer, then convert once, apply 2^(ea + eb), pair the
+// of each operand a stage) into a 3-stage shared-memory ring; one thread issues tcgen05.mma (M = 128, N = 256 or 128,
+// K = 16, bf16 in, FP32 out) into four 128-column tensor-memory accumulators; eight warps read each finished
+// accumulator out of tensor memory (tcgen05.ld) and add it, as an integer at its diagonal's weight, into one int64 per
+// element while the next group accumulates in other slots, then convert once, apply 2^(ea + eb), pair the
 // real and imaginary rows and write C. Every mbarrier wait is bounded: on expiry the kernel records an error,
 // drains its own copies and products, frees its tensor memory and returns without writing C.
+//
+// Shared memory bounds the products: an MMA of N = 128 reads 8 KB of operands in the 64 cycles it takes, 128 bytes a
+// cycle, all there is, and the copies write there too. So digits go in quads, two of A and two of B a stage: four
+// digit products for four boxes instead of two, and A_i meets both of B's in one MMA of N = 256 (12 KB in 128 cycles).
+// Order 121: a pair and 128 K a stage took 1430 cycles a stage (80,000 a tile), quads with N = 128 MMAs 1575 (68,000, at
+// 125 bytes a cycle); 4096 products with their digit splits 4.65, 4.39 and, with N = 256, 4.27 ms; 64 of order 301
+// 0.856, 0.831, 0.766. With K = 32 (the factorisations' updates) all three take 1.85: loads and conversion bound those.
 #include <cuda.h>
 #include <cuda_runtime.h>
 
@@ -50,24 +57,29 @@ constexpr int kStageBoxes = 2;
 constexpr int kStages = 3;
 constexpr int kBoxBytes = kTileM * kTileK * 2;               // 16 KB
 constexpr int kStageBytes = 2 * kStageBoxes * kBoxBytes;      // A boxes, then B boxes: 64 KB
-constexpr int kTmemCols = 256;                                // two accumulators of 128 columns
+constexpr int kSlots = 4;                                     // accumulators of 128 tensor-memory columns
+constexpr int kTmemCols = kSlots * kTileN;
 constexpr int kThreads = 320;                                 // producer, MMA, 8 epilogue warps
 constexpr int kMaxGroups = 160;
 constexpr int kMaxSlices = 8;
 constexpr unsigned kWaitLimit = 1u << 22;  // try_wait rounds before a wait is declared stuck
 
-// One accumulation group: digit pairs (i, d - i) for i in [i0, i0 + ni), K blocks [kb0, kb0 + nkb).
+// One accumulation group over K blocks [kb0, kb0 + nkb). Quads: for p < ni, i = i0 + 2 p, j = d - i, the digit pairs
+// (i, j), (i, j + 1), (i + 1, j), (i + 1, j + 1), into three accumulators (diagonals d, d + 1, d + 2). Singles: the
+// pairs (i, d - i), i = i0 + step p, into one; step 2 on even diagonals, where quads hold the pairs between.
 struct Plan {
     int n_groups;
     int S;
     int s0;  // the int64 accumulator holds the product in units of 2^(-14 - s0) (diagonal d enters times 2^(s0 - 8 (d - 2)))
-    unsigned g[kMaxGroups];  // d | i0 << 4 | ni << 8 | kb0 << 12 | nkb << 22
+    unsigned g[kMaxGroups];  // d | i0 << 4 | ni << 8 | kb0 << 12 | nkb << 22 | quads << 31
 };
 __host__ __device__ inline int g_d(unsigned v) { return v & 15; }
 __host__ __device__ inline int g_i0(unsigned v) { return (v >> 4) & 15; }
 __host__ __device__ inline int g_ni(unsigned v) { return (v >> 8) & 15; }
 __host__ __device__ inline int g_kb0(unsigned v) { return (v >> 12) & 1023; }
-__host__ __device__ inline int g_nkb(unsigned v) { return (v >> 22) & 1023; }
+__host__ __device__ inline int g_nkb(unsigned v) { return (v >> 22) & 511; }
+__host__ __device__ inline bool g_quad(unsigned v) { return v >> 31; }
+__host__ __device__ inline int g_step(unsigned v) { return 2 - (int)(v & 1u); }
 
 // ---------------------------------------------------------------- PTX wrappers
 
@@ -124,13 +136,14 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr) {
            ((uint64_t)2 << 61);
 }
 
-// instruction descriptor: D f32, A and B bf16, both K-major, N = 128, M = 128
-constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kTileN >> 3) << 17) | ((uint32_t)(kTileM >> 4) << 24);
+// instruction descriptor: D f32, A and B bf16, both K-major, M = 128
+__host__ __device__ constexpr uint32_t mma_idesc(int n) { return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kTileM >> 4) << 24); }
 
+template <int N>
 __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t accumulate) {
     asm volatile(
         "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(d_tmem),
-        "l"(adesc), "l"(bdesc), "r"(kIdesc), "r"(accumulate)
+        "l"(adesc), "l"(bdesc), "r"(mma_idesc(N)), "r"(accumulate)
         : "memory");
 }
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
@@ -448,8 +461,21 @@ __device__ __forceinline__ double finish_element(long long ac, int e, int s0, lo
     return __hiloint2double(a == 0 ? 0 : hi, a == 0 ? 0 : (int)q);
 }
 
+// The accumulator slots of the next group (quads and singles count the groups of each kind so far). Quads need their
+// three diagonals in neighbouring columns, the middle one between; they take slots 0 1 2 and 3 2 1 in turn (the
+// second with B's boxes exchanged), so that their first products need one slot of the group before, the one that is
+// drained first.
+struct GroupSlots {
+    int low, mid, high;
+};
+__device__ __forceinline__ GroupSlots group_slots(bool quad, int& quads, int& singles) {
+    if (quad) return quads++ & 1 ? GroupSlots{3, 2, 1} : GroupSlots{0, 1, 2};
+    const int s = singles++ & 1 ? 0 : 3;
+    return GroupSlots{s, s, s};
+}
+
 struct SharedState {
-    uint64_t full[kStages], empty[kStages], tfull[2], tempty[2], drain;
+    uint64_t full[kStages], empty[kStages], tfull[kSlots], tempty[kSlots], drain;
     uint32_t tmem_base;
     int abort_flag;
     int eb[kTileN];  // the columns' scale exponents
@@ -494,7 +520,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             mbar_init(&ss->full[s], 1);
             mbar_init(&ss->empty[s], 1);
         }
-        for (int s = 0; s < 2; ++s) {
+        for (int s = 0; s < kSlots; ++s) {
             mbar_init(&ss->tfull[s], 1);
             mbar_init(&ss->tempty[s], 8);
         }
@@ -522,27 +548,31 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (warp == 0) {
         // ---- TMA producer
         if (lane == 0) {
-            int st = 0, ph = 1, issued = 0;
+            int st = 0, ph = 1, issued = 0, quads = 0;
             bool ok = true;
             for (int gi = 0; gi < plan.n_groups && ok; ++gi) {
                 const unsigned g = plan.g[gi];
                 const int d = g_d(g), i0 = g_i0(g), ni = g_ni(g), kb0 = g_kb0(g), kb1 = kb0 + g_nkb(g);
+                const bool quad = g_quad(g);
+                const int step = quad ? 2 : g_step(g), flip = quad ? quads++ & 1 : 0;
                 for (int p = 0; p < ni && ok; ++p) {
-                    const int pa = za * S + i0 + p - 1, pb = zb * S + d - i0 - p - 1;
-                    for (int kb = kb0; kb < kb1; kb += kStageBoxes) {
+                    const int i = i0 + step * p, pa = za * S + i - 1, pb = zb * S + d - i - 1;
+                    for (int kb = kb0; kb < kb1; kb += quad ? 1 : kStageBoxes) {
                         if (!mbar_wait(&ss->empty[st], ph, abort_flag, err)) {
                             ok = false;
                             break;
                         }
                         unsigned char* sa = smem + st * kStageBytes;
                         uint64_t* full = &ss->full[st];
-                        const bool two = kb + 1 < kb1;
+                        // the second box of each operand: the next digit, or the next K block
+                        const int kn = quad ? kb : kb + 1, dn = quad ? 1 : 0;
+                        const bool two = quad || kb + 1 < kb1;
                         mbar_expect_tx(full, two ? kStageBytes : kStageBytes / 2);
                         tma_load_3d(sa, &map_a, kb * kTileK, m0, pa, full);
-                        tma_load_3d(sa + kStageBoxes * kBoxBytes, &map_b, kb * kTileK, n0, pb, full);
+                        tma_load_3d(sa + kStageBoxes * kBoxBytes, &map_b, kb * kTileK, n0, pb + flip, full);
                         if (two) {
-                            tma_load_3d(sa + kBoxBytes, &map_a, (kb + 1) * kTileK, m0, pa, full);
-                            tma_load_3d(sa + (kStageBoxes + 1) * kBoxBytes, &map_b, (kb + 1) * kTileK, n0, pb, full);
+                            tma_load_3d(sa + kBoxBytes, &map_a, kn * kTileK, m0, pa + dn, full);
+                            tma_load_3d(sa + (kStageBoxes + 1) * kBoxBytes, &map_b, kn * kTileK, n0, pb + dn - flip, full);
                         }
                         ++issued;
                         if (++st == kStages) {
@@ -566,39 +596,69 @@ __global__ void __launch_bounds__(kThreads, 1)
         // ---- MMA issuer
         if (lane == 0) {
             const uint64_t base = smem_desc_sw128(smem_u32(smem));
-            int st = 0, ph = 0;
+            int st = 0, ph = 0, quads = 0, singles = 0;
+            uint32_t used = 0;  // a bit per slot: the parity of its uses so far
             bool ok = true;
             bool any = false;
+            const auto slot_free = [&](int slot) {
+                if (!mbar_wait(&ss->tempty[slot], (used >> slot & 1) ^ 1, abort_flag, err)) return false;
+                used ^= 1u << slot;
+                return true;
+            };
+            const auto slot_cols = [&](int slot) { return tmem + slot * kTileN; };
+            // the four MMAs of one box of A and one of B; descriptors count 16-byte units: 32 bytes of K further is + 2
+            const auto box_mma = [&](uint32_t d_tmem, uint64_t da, uint64_t db, uint32_t acc) {
+#pragma unroll
+                for (int kk = 0; kk < kTileK / 16; ++kk) mma_bf16<kTileN>(d_tmem, da + 2 * kk, db + 2 * kk, kk ? 1u : acc);
+            };
+            constexpr uint64_t box = kBoxBytes >> 4;
             for (int gi = 0; gi < plan.n_groups && ok; ++gi) {
                 const unsigned g = plan.g[gi];
-                const int buf = gi & 1, ni = g_ni(g), nkb = g_nkb(g);
-                if (!mbar_wait(&ss->tempty[buf], ((gi >> 1) & 1) ^ 1, abort_flag, err)) {
-                    ok = false;
-                    break;
-                }
-                tc_fence_after();
-                const uint32_t d_tmem = tmem + buf * kTileN;
+                const int ni = g_ni(g), nkb = g_nkb(g);
+                const bool quad = g_quad(g);
+                const GroupSlots gs = group_slots(quad, quads, singles);
                 uint32_t acc = 0;
                 for (int p = 0; p < ni && ok; ++p) {
-                    for (int kb = 0; kb < nkb; kb += kStageBoxes) {
+                    for (int kb = 0; kb < nkb; kb += quad ? 1 : kStageBoxes) {
                         if (!mbar_wait(&ss->full[st], ph, abort_flag, err)) {
                             ok = false;
                             break;
                         }
+                        // a slot is waited for when its first product is about to be issued
+                        if (!acc && !(slot_free(gs.low) && (!quad || slot_free(gs.mid)))) {
+                            ok = false;
+                            break;
+                        }
                         tc_fence_after();
-                        // descriptors count 16-byte units: 32 bytes of K further is + 2, a box is + 1024
-                        const uint64_t da = base + (uint64_t)st * (kStageBytes >> 4), db = da + (kStageBoxes * kBoxBytes >> 4);
-#pragma unroll
-                        for (int kk = 0; kk < kTileK / 16; ++kk) {
-                            mma_bf16(d_tmem, da + 2 * kk, db + 2 * kk, acc);
-                            acc = 1;
-                        }
-                        if (kb + 1 < nkb) {
-#pragma unroll
-                            for (int kk = 0; kk < kTileK / 16; ++kk)
-                                mma_bf16(d_tmem, da + (kBoxBytes >> 4) + 2 * kk, db + (kBoxBytes >> 4) + 2 * kk, 1);
-                        }
+                        const uint64_t a0 = base + (uint64_t)st * (kStageBytes >> 4), b0 = a0 + kStageBoxes * box;
                         any = true;
+                        if (quad) {
+                            // A_i by both boxes of B: diagonals d and d + 1, side by side
+                            const uint32_t d0 = slot_cols(min(gs.low, gs.mid)), d1 = slot_cols(min(gs.mid, gs.high));
+#pragma unroll
+                            for (int kk = 0; kk < kTileK / 16; ++kk) mma_bf16<2 * kTileN>(d0, a0 + 2 * kk, b0 + 2 * kk, kk ? 1u : acc);
+                            if (!acc) {
+                                if (!slot_free(gs.high)) {
+                                    ok = false;
+                                    break;
+                                }
+                                tc_fence_after();
+                            }
+                            // A_(i+1): diagonals d + 1 and d + 2, the first of d + 2 on its own
+                            const uint64_t a1 = a0 + box;
+                            if (acc) {
+                                mma_bf16<2 * kTileN>(d1, a1, b0, 1);
+                            } else {
+                                mma_bf16<kTileN>(d1, a1, b0, gs.mid < gs.high);
+                                mma_bf16<kTileN>(d1 + kTileN, a1, b0 + box, gs.mid > gs.high);
+                            }
+#pragma unroll
+                            for (int kk = 1; kk < kTileK / 16; ++kk) mma_bf16<2 * kTileN>(d1, a1 + 2 * kk, b0 + 2 * kk, 1);
+                        } else {
+                            box_mma(slot_cols(gs.low), a0, b0, acc);
+                            if (kb + 1 < nkb) box_mma(slot_cols(gs.low), a0 + box, b0 + box, 1);
+                        }
+                        acc = 1;
                         mma_commit(&ss->empty[st]);  // the stage is free once these products have read it
                         if (++st == kStages) {
                             st = 0;
@@ -606,7 +666,13 @@ __global__ void __launch_bounds__(kThreads, 1)
                         }
                     }
                 }
-                if (ok) mma_commit(&ss->tfull[buf]);
+                if (ok) {
+                    mma_commit(&ss->tfull[gs.low]);
+                    if (quad) {
+                        mma_commit(&ss->tfull[gs.mid]);
+                        mma_commit(&ss->tfull[gs.high]);
+                    }
+                }
             }
             if (!ok && any) {
                 // drain: every product issued so far completes before the accumulators are freed
@@ -628,13 +694,23 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
         for (int c = 0; c < 64; ++c) acc[c] = 0;
         bool ok = true;
-        for (int gi = 0; gi < plan.n_groups; ++gi) {
-            const int buf = gi & 1;
-            ok = mbar_wait(&ss->tfull[buf], (gi >> 1) & 1, abort_flag, err);
+        int quads = 0, singles = 0;
+        uint32_t used = 0;
+        GroupSlots gs{};
+        for (int gi = 0, part = -1; gi < plan.n_groups;) {
+            const unsigned g = plan.g[gi];
+            if (part < 0) {
+                gs = group_slots(g_quad(g), quads, singles);
+                part = g_quad(g) ? 2 : 0;
+            }
+            // the highest diagonal first: its slot is the first that the next quads need
+            const int buf = part == 2 ? gs.high : part == 1 ? gs.mid : gs.low;
+            ok = mbar_wait(&ss->tfull[buf], used >> buf & 1, abort_flag, err);
+            used ^= 1u << buf;
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             tc_fence_after();
-            const int sh = plan.s0 - 8 * (g_d(plan.g[gi]) - 2);
+            const int sh = plan.s0 - 8 * (g_d(g) + part - 2);
             const uint32_t base = tmem + ((uint32_t)(q * 32) << 16) + buf * kTileN + h * 64;
             float v[32];
             tmem_ld32(base, v);
@@ -644,6 +720,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             __syncwarp();
             if (lane == 0) mbar_arrive(&ss->tempty[buf]);
             add_group(acc + 32, v, sh);
+            if (--part < 0) ++gi;
         }
         if (ok && !*abort_flag) {
             // Each lane writes its own row's part of C: row r of C^ is the real (r even) or imaginary part of
@@ -730,28 +807,32 @@ CUtensorMap plane_map(const uint16_t* base, long long rows, int Kp, long long pl
     return map;
 }
 
-// The groups, smallest contributions first: diagonal d = S + 1 down to 2, K in chunks of at most 1024,
-// at most 1024 / (chunk length) digit pairs per group so every group's sum is exact in FP32.
+// The groups, smallest contributions first: the single pairs that quads leave (the odd i of the even one of diagonals
+// S and S + 1, and all of diagonal S + 1 where S is even), then the quads by their first diagonal. Every accumulator's
+// sum is exact in FP32: at most 1024 digit products, so K in chunks of at most 1024 (quads, whose middle diagonal takes
+// two pairs each: 512) and as many pairs a group as that leaves.
 Plan make_plan(int S, int kblocks) {
     Plan p{};
     p.S = S;
     int lg = 0;
     while ((1 << lg) < kblocks * kTileK) ++lg;
     p.s0 = 47 - lg;
-    const int chunk_kb = 1024 / kTileK;
-    for (int d = S + 1; d >= 2; --d) {
-        const int lo = std::max(1, d - S), hi = std::min(S, d - 1);
-        for (int kb0 = 0; kb0 < kblocks; kb0 += chunk_kb) {
-            const int nkb = std::min(chunk_kb, kblocks - kb0);
-            const int per = std::max(1, 1024 / (nkb * kTileK));
-            for (int i0 = lo; i0 <= hi; i0 += per) {
+    const auto add = [&](bool quad, int d, int lo, int hi) {  // i = lo, lo + step .. hi
+        const int step = quad ? 2 : 2 - (d & 1), most = 1024 / kTileK / (quad ? 2 : 1);
+        for (int kb0 = 0; kb0 < kblocks; kb0 += most) {
+            const int nkb = std::min(most, kblocks - kb0), per = std::max(1, most / nkb);
+            for (int i0 = lo; i0 <= hi; i0 += step * per) {
                 if (p.n_groups >= kMaxGroups) throw EngineError{RCWA_EUNSUPPORTED, "tensor-core GEMM: K too large"};
-                const int ni = std::min(per, hi - i0 + 1);
-                p.g[p.n_groups++] = (unsigned)d | (unsigned)i0 << 4 | (unsigned)ni << 8 | (unsigned)kb0 << 12 |
-                                    (unsigned)nkb << 22;
+                const int ni = std::min(per, (hi - i0) / step + 1);
+                p.g[p.n_groups++] = (unsigned)d | (unsigned)i0 << 4 | (unsigned)ni << 8 | (unsigned)kb0 << 12 | (unsigned)nkb << 22 |
+                                    (quad ? 1u << 31 : 0u);
             }
         }
-    }
+    };
+    if (S % 2 == 0) add(false, S + 1, 1, S);
+    const int even = S % 2 ? S + 1 : S;
+    add(false, even, 1, even - 1);
+    for (int d = even - 2; d >= 2; d -= 2) add(true, d, 1, d - 1);
     return p;
 }
 
