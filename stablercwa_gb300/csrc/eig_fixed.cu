@@ -114,9 +114,15 @@ void launch_herm_reduce_fixed(cudaStream_t st, int n, int batch, const zc* a, lo
 }
 
 void launch_herm_ql_fixed(cudaStream_t st, int n, int batch, zc* w, int* info, zc* ws, const int* status) {
-    const size_t smem = (size_t)2 * n * kHermQlThreads * sizeof(long long);
+    // A matrix a lane, and no more lanes a warp than give each SM one warp: lanes of a warp run sweeps of different
+    // lengths, and the chain of one waits for the branches of the others (16 matrices of order 301: 65 ms in one warp,
+    // 50 in a warp each; the scan of them 152 to 137 ms). One warp a scheduler (608 in all) leaves the other polarisation's stream less room: the
+    // mirror sweep, 4096 matrices a stream, 381 against 372 ms.
+    int lanes = 1;
+    while (lanes < kHermQlThreads && 152LL * lanes < batch) lanes *= 2;
+    const size_t smem = (size_t)2 * n * lanes * sizeof(long long);
     if (smem > 48 * 1024) ensure_smem_optin(reinterpret_cast<const void*>(herm_ql_fixed_kernel), (int)smem);
-    herm_ql_fixed_kernel<<<(unsigned)((batch + kHermQlThreads - 1) / kHermQlThreads), kHermQlThreads, smem, st>>>(
+    herm_ql_fixed_kernel<<<(unsigned)((batch + lanes - 1) / lanes), lanes, smem, st>>>(
         n, batch, w, info, ws, status, rotation_counter());
     RCWA_CUDA(cudaGetLastError());
 }

@@ -1043,8 +1043,8 @@ static __global__ void __launch_bounds__(kHermQlThreads) herm_ql_fixed_kernel(in
     const double* src = reinterpret_cast<const double*>(base + 2LL * n * n);
     int* tail = reinterpret_cast<int*>(base + 3LL * n * n);  // [0] sweeps, [1] left to the fused kernel
     long long* d = fixq_sm + threadIdx.x;
-    long long* e = d + (long long)n * kHermQlThreads;
-    constexpr int sd = kHermQlThreads;
+    const int sd = blockDim.x;
+    long long* e = d + n * sd;
     // the scale
     float big = 0.0f;
     int e2 = 0;
