@@ -21,6 +21,27 @@ constexpr long long kFixLogBytes = 4LL << 30;
 // what shared memory holds), at least four so that three warps trail the one that forms the rotations
 int fix_warps(int n) { return std::min(11, std::max(4, (n + 31) / 32)); }
 
+// Rows a CTA of the log's application: 32, or 16 where shared memory holds one CTA of 32 rows an SM (order 222 on) and
+// they are more than the SMs: two CTAs of 16 take an SM in the time of one of 32 (a chain of latencies). 16 matrices of
+// order 301, 160 CTAs of 32 rows on 152 SMs: the order-301
+// scan 136.6 to 132.5 ms.
+template <int R>
+void fix_apply_rows(cudaStream_t st, int n, int batch, zc* z, long long z_stride, const int4* log, long long log_stride,
+                    const int4* table, const int* head, const int* status) {
+    const size_t smem = (size_t)n * R * sizeof(lz);
+    if (smem > 45 * 1024) ensure_smem_optin(reinterpret_cast<const void*>(fix_apply_kernel<R>), (int)smem);
+    fix_apply_kernel<R><<<dim3((unsigned)batch, (unsigned)((n + R - 1) / R)), R, smem, st>>>(n, batch, z, z_stride, log, log_stride, table,
+                                                                                            head, status);
+    RCWA_CUDA(cudaGetLastError());
+}
+void fix_apply(cudaStream_t st, int n, int batch, zc* z, long long z_stride, const int4* log, long long log_stride, const int4* table,
+               const int* head, const int* status) {
+    if (n >= 222 && (long long)batch * ((n + 31) / 32) > 152)
+        fix_apply_rows<16>(st, n, batch, z, z_stride, log, log_stride, table, head, status);
+    else
+        fix_apply_rows<32>(st, n, batch, z, z_stride, log, log_stride, table, head, status);
+}
+
 }  // namespace
 
 // RCWA_GB300_EIG_FIXED=0 keeps the FP64 iterations
@@ -43,10 +64,8 @@ void launch_eig_fixed(cudaStream_t st, int n, int batch, const zc* a, long long 
                       int* done, double eps, zc* t_out) {
     const long long nn = (long long)n * n, wst = (3 * nn + 4LL * n + 8);  // eig_workspace_elems
     const int warps = fix_warps(n);
-    const size_t schur_smem = fix_schur_smem(n, warps), row_smem = (size_t)n * 32 * sizeof(lz),
-                 back_smem = (size_t)(n + 4) * 32 * sizeof(zc);
+    const size_t schur_smem = fix_schur_smem(n, warps), back_smem = (size_t)(n + 4) * 32 * sizeof(zc);
     ensure_smem_optin(reinterpret_cast<const void*>(fix_schur_kernel<false>), (int)schur_smem);
-    if (row_smem > 45 * 1024) ensure_smem_optin(reinterpret_cast<const void*>(fix_apply_kernel), (int)row_smem);
     if (back_smem > 48 * 1024) ensure_smem_optin(reinterpret_cast<const void*>(fix_backsub_kernel), (int)back_smem);
     const int chunk = (int)std::max(1LL, std::min<long long>(std::min(batch, std::max(kFixPassMin, (batch + 1) / 2)),
                                                              kFixLogBytes / eig_fixed_bytes(n)));
@@ -67,9 +86,7 @@ void launch_eig_fixed(cudaStream_t st, int n, int batch, const zc* a, long long 
         fix_schur_kernel<false><<<(unsigned)cb, 32 * warps, schur_smem, st>>>(n, cb, ac, a_stride, wc, h, wst, log, 2 * fix_log_capacity(n), table, head, status,
                                                                        done + b0, info + b0);
         RCWA_CUDA(cudaGetLastError());
-        fix_apply_kernel<<<dim3((unsigned)cb, (unsigned)((n + 31) / 32)), 32, row_smem, st>>>(n, cb, z1, wst, log, 2 * fix_log_capacity(n), table,
-                                                                                               head, status);
-        RCWA_CUDA(cudaGetLastError());
+        fix_apply(st, n, cb, z1, wst, log, 2 * fix_log_capacity(n), table, head, status);
         zc* t = t_out ? t_out + (long long)b0 * nn : vc;
         RCWA_CUDA(cudaMemsetAsync(tn, 0, (size_t)cb * sizeof(unsigned long long), st));
         fix_triangle_kernel<<<(unsigned)((nn * cb + 255) / 256), 256, 0, st>>>(n, cb, h, wst, t, nn, wc, head, status, tn);
@@ -95,9 +112,8 @@ void launch_eig_fixed(cudaStream_t st, int n, int batch, const zc* a, long long 
 void launch_herm_reduce_fixed(cudaStream_t st, int n, int batch, const zc* a, long long a_stride, zc* q, zc* ws, int* status) {
     const long long nn = (long long)n * n, wst = 3 * nn + 4LL * n + 8, log_stride = 2 * fix_reduce_capacity(n);
     const int warps = fix_warps(n);
-    const size_t schur_smem = fix_schur_smem(n, warps), row_smem = (size_t)n * 32 * sizeof(lz);
+    const size_t schur_smem = fix_schur_smem(n, warps);
     ensure_smem_optin(reinterpret_cast<const void*>(fix_schur_kernel<true>), (int)schur_smem);
-    if (row_smem > 45 * 1024) ensure_smem_optin(reinterpret_cast<const void*>(fix_apply_kernel), (int)row_smem);
     int4* log = nullptr;
     int* head = nullptr;
     RCWA_CUDA(cudaMallocAsync(&log, (size_t)batch * log_stride * sizeof(int4), st));
@@ -105,9 +121,7 @@ void launch_herm_reduce_fixed(cudaStream_t st, int n, int batch, const zc* a, lo
     fix_schur_kernel<true><<<(unsigned)batch, 32 * warps, schur_smem, st>>>(n, batch, a, a_stride, nullptr, reinterpret_cast<lz*>(ws), wst,
                                                                             log, log_stride, nullptr, head, status, nullptr, nullptr);
     RCWA_CUDA(cudaGetLastError());
-    fix_apply_kernel<<<dim3((unsigned)batch, (unsigned)((n + 31) / 32)), 32, row_smem, st>>>(n, batch, q, nn, log, log_stride, nullptr, head,
-                                                                                             status);
-    RCWA_CUDA(cudaGetLastError());
+    fix_apply(st, n, batch, q, nn, log, log_stride, nullptr, head, status);
     launch_count() += 2;
     RCWA_CUDA(cudaFreeAsync(log, st));
     RCWA_CUDA(cudaFreeAsync(head, st));

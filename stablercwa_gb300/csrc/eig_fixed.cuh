@@ -770,35 +770,41 @@ __global__ void fix_schur_kernel(int n, int batch, const zc* __restrict__ a_in, 
     }
 }
 
-// Z from the log: a lane per row, 32 rows a CTA, the row in shared memory (row t of the CTA at element
-// i * 32 + t). A similarity H <- G H G^H takes Z <- Z G^H: (a', b') = (q a + s b, conj(q) b - s a).
-static __global__ void __launch_bounds__(32) fix_apply_kernel(int n, int batch, zc* __restrict__ z_out, long long z_stride,
+// Z from the log: a lane per row, R rows (and lanes) a CTA, the row in shared memory (row t of the CTA at element
+// i * R + t). A similarity H <- G H G^H takes Z <- Z G^H: (a', b') = (q a + s b, conj(q) b - s a).
+template <int R = 32>
+__global__ void __launch_bounds__(R) fix_apply_kernel(int n, int batch, zc* __restrict__ z_out, long long z_stride,
                                                               const int4* __restrict__ log_all, long long log_stride,
                                                               const int4* __restrict__ table_all, const int* __restrict__ head, const int* __restrict__ status) {
     RCWA_DYN_SMEM(lz, fixz_sm);
     const long long gid = blockIdx.x;
-    const int lane = threadIdx.x, row = blockIdx.y * 32 + lane;
+    const int lane = threadIdx.x, row = blockIdx.y * R + lane;
     if (gid >= batch || status[gid]) return;
     lz* y = fixz_sm + lane;
-    for (int i = 0; i < n; ++i) y[i * 32] = lz{i == row ? 1LL << 60 : 0, 0};
+    for (int i = 0; i < n; ++i) y[i * R] = lz{i == row ? 1LL << 60 : 0, 0};
     // the log through shared memory: chunk c (32 rotations) in stage[c & 1], the next in registers on its way.
     // Runs of rotations are cut at the chunks' ends, so that nothing inside a run depends on the staging.
     __shared__ int4 stage[2][68];  // a run reads one rotation past its end
     const int4* log = log_all + gid * log_stride + lane;
     const int4* table = table_all + gid * fix_table_capacity(n);
-    stage[0][lane] = log[0];
-    stage[0][lane + 32] = log[32];
-    int4 n0 = log[64], n1 = log[96];
+    constexpr int kLoads = 64 / R;  // of a chunk's int4s, a lane
+    int4 nx[kLoads];
+#pragma unroll
+    for (int u = 0; u < kLoads; ++u) {
+        stage[0][lane + u * R] = log[u * R];
+        nx[u] = log[64 + u * R];
+    }
     log += 128;
     const int4* e = stage[0];
     int left = 32, b = 0;  // rotations left in the chunk
     __syncwarp();
     const auto refill = [&] {
         b ^= 1;
-        stage[b][lane] = n0;
-        stage[b][lane + 32] = n1;
-        n0 = log[0];
-        n1 = log[32];
+#pragma unroll
+        for (int u = 0; u < kLoads; ++u) {
+            stage[b][lane + u * R] = nx[u];
+            nx[u] = log[u * R];
+        }
         log += 64;
         e = stage[b];
         left = 32;
@@ -815,22 +821,22 @@ static __global__ void __launch_bounds__(32) fix_apply_kernel(int n, int batch, 
         const int m = n - 1 - k, len = fix_seg_len(m), ns = (m + len - 1) / len, top_row = k + 1;
         for (int sg = 0; sg < ns; ++sg) {
             const int t0 = top_row + sg * len, t1 = min(t0 + len, n);
-            lz v = fix_phase<true>(next(), y[(t1 - 1) * 32]);
-            lz x = y[max(t1 - 2, t0) * 32];
+            lz v = fix_phase<true>(next(), y[(t1 - 1) * R]);
+            lz x = y[max(t1 - 2, t0) * R];
             for (int i = t1 - 2; i >= t0; --i) {
-                const lz xn = y[max(i - 1, t0) * 32];
+                const lz xn = y[max(i - 1, t0) * R];
                 lz oa, ob;
                 fix_pair<true>(next(), x, v, oa, ob);
-                y[(i + 1) * 32] = ob;
+                y[(i + 1) * R] = ob;
                 v = oa;
                 x = xn;
             }
-            y[t0 * 32] = v;
+            y[t0 * R] = v;
         }
         for (int d = 1; d < ns; d *= 2)
             for (int sg = 0; sg + d < ns; sg += 2 * d) {
-                lz* pa = y + (top_row + sg * len) * 32;
-                lz* pb = y + (top_row + (sg + d) * len) * 32;
+                lz* pa = y + (top_row + sg * len) * R;
+                lz* pb = y + (top_row + (sg + d) * len) * R;
                 lz oa, ob;
                 fix_pair<true>(next(), *pa, *pb, oa, ob);
                 *pa = oa;
@@ -840,31 +846,31 @@ static __global__ void __launch_bounds__(32) fix_apply_kernel(int n, int batch, 
     const int sweeps = head[2 * gid];
     for (int k = 0; k < sweeps; ++k) {
         const int4 tb = table[k];
-        lz* p = y + tb.x * 32;
-        lz v = p[0], z = p[32];
+        lz* p = y + tb.x * R;
+        lz v = p[0], z = p[R];
         for (int todo = tb.y - tb.x; todo > 0;) {
             if (left == 0) refill();
             const int run = min(todo, left);
             int4 u0 = e[0], v0 = e[1];
             for (int q = 0; q < run; q += 2) {  // two a turn, each one's coefficients and entry read a turn ahead
                 const int4 u1 = e[2], v1 = e[3];
-                const lz z1 = p[todo - q < 2 ? 32 : 2 * 32];
+                const lz z1 = p[todo - q < 2 ? R : 2 * R];
                 lz oa, ob;
                 fix_pair<true>(fix_log_get(u0, v0), v, z, oa, ob);
                 p[0] = oa;
                 v = ob;
                 z = z1;
-                p += 32;
+                p += R;
                 e += 2;
                 if (q + 1 == run) break;
                 u0 = e[2];
                 v0 = e[3];
-                const lz z2 = p[todo - q - 1 < 2 ? 32 : 2 * 32];
+                const lz z2 = p[todo - q - 1 < 2 ? R : 2 * R];
                 fix_pair<true>(fix_log_get(u1, v1), v, z, oa, ob);
                 p[0] = oa;
                 v = ob;
                 z = z2;
-                p += 32;
+                p += R;
                 e += 2;
             }
             todo -= run;
@@ -875,7 +881,7 @@ static __global__ void __launch_bounds__(32) fix_apply_kernel(int n, int batch, 
     }
     if (row >= n) return;
     zc* zo = z_out + gid * z_stride + row;
-    for (int i = 0; i < n; ++i) zo[(long long)i * n] = zc{(double)y[i * 32].re * 0x1p-60, (double)y[i * 32].im * 0x1p-60};
+    for (int i = 0; i < n; ++i) zo[(long long)i * n] = zc{(double)y[i * R].re * 0x1p-60, (double)y[i * R].im * 0x1p-60};
 }
 
 // The Schur form from the reduced matrix h (lz): its upper triangle, the eigenvalues on the diagonal, zeros below;
