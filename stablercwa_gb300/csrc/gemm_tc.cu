@@ -33,7 +33,7 @@
 // digit products for four boxes instead of two, and A_i meets both of B's in one MMA of N = 256 (12 KB in 128 cycles).
 // Order 121: a pair and 128 K a stage took 1430 cycles a stage (80,000 a tile), quads with N = 128 MMAs 1575 (68,000, at
 // 125 bytes a cycle); 4096 products with their digit splits 4.65, 4.39 and, with N = 256, 4.27 ms; 64 of order 301
-// 0.856, 0.831, 0.766. With K = 32 (the factorisations' updates) all three take 1.85: loads and conversion bound those.
+// 0.856, 0.831, 0.766. With K = 32 (the factorisations' updates) the three are equal: loads and the conversion bound those.
 #include <cuda.h>
 #include <cuda_runtime.h>
 
@@ -42,6 +42,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "engine.h"
@@ -440,11 +441,10 @@ __device__ __noinline__ double finish_slow(long long ac, int e, int s0, double c
     return fma(s_c, c0, s_ab * ldexp((double)ac, e - 14 - s0));
 }
 template <bool HasC0>
-__device__ __forceinline__ double finish_element(long long ac, int e, int s0, long long neg, bool unit_scales, double c0, double s_ab,
-                                                 double s_c) {
+__device__ __forceinline__ double finish_fast(long long ac, int e, int s0, long long neg, bool unit_scales, double c0, bool& fast) {
     const int e2 = e - 14 - s0;
     long long a = (ac ^ neg) - neg;  // neg: 0 or -1
-    bool fast = unit_scales;
+    fast = unit_scales;
     if (HasC0) {
         long long t;
         fast = double_to_units(c0, e2, t) && fast;
@@ -456,9 +456,36 @@ __device__ __forceinline__ double finish_element(long long ac, int e, int s0, lo
     const unsigned long long q = (w + 0x1FF + ((unsigned)(w >> 10) & 1u)) >> 10;  // 53 bits, or 2^53: the sum below carries it
     const int ex = 1085 - lz + e2;  // biased exponent - 1
     fast = fast && (a == 0 ? e < kNonFinite / 2 : (unsigned)ex < 2045u);
-    if (!fast) return finish_slow(ac, e, s0, HasC0 ? c0 : 0.0, s_ab, HasC0 ? s_c : 0.0);
     const int hi = (int)(q >> 32) + (ex << 20) + (a < 0 ? (int)0x80000000 : 0);
     return __hiloint2double(a == 0 ? 0 : hi, a == 0 ? 0 : (int)q);
+}
+// Four elements at once, their rare cases after all of them: with a branch an element nothing of the next one
+// started before the last was done, and two warps a scheduler do not hide that (4096 products of order 121
+// with their splits 4.27 to 4.14 ms, of 121 x 32 x 121 1.88 to 1.70, of order 81 3.02 to 2.83).
+template <bool HasC0>
+__device__ __forceinline__ void finish_four(const long long* ac, const int* e, int s0, long long neg, bool unit_scales, const double* c0,
+                                            double s_ab, double s_c, double* out) {
+    bool fast[4], all = true;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        out[u] = finish_fast<HasC0>(ac[u], e[u], s0, neg, unit_scales, HasC0 ? c0[u] : 0.0, fast[u]);
+        all = all && fast[u];
+    }
+    if (!all) {
+#pragma unroll 1
+        for (int u = 0; u < 4; ++u) {
+            const bool f = u == 0 ? fast[0] : u == 1 ? fast[1] : u == 2 ? fast[2] : fast[3];
+            if (f) continue;
+            const long long a = u == 0 ? ac[0] : u == 1 ? ac[1] : u == 2 ? ac[2] : ac[3];
+            const int ee = u == 0 ? e[0] : u == 1 ? e[1] : u == 2 ? e[2] : e[3];
+            const double c = !HasC0 ? 0.0 : u == 0 ? c0[0] : u == 1 ? c0[1] : u == 2 ? c0[2] : c0[3];
+            const double r = finish_slow(a, ee, s0, c, s_ab, HasC0 ? s_c : 0.0);
+            if (u == 0) out[0] = r;
+            else if (u == 1) out[1] = r;
+            else if (u == 2) out[2] = r;
+            else out[3] = r;
+        }
+    }
 }
 
 // The accumulator slots of the next group (quads and singles count the groups of each kind so far). Quads need their
@@ -746,22 +773,26 @@ __global__ void __launch_bounds__(kThreads, 1)
                 const int* se = ss->eb + h * 64;
                 const long long step = 2LL * ldc, neg = s_ab < 0.0 ? -1 : 0;
                 long long off2 = 2 * ((long long)(n0 + h * 64) * ldc + i) + part;
-                if (C0d) {
+                const auto finish = [&](auto has_c0) {
+                    constexpr bool kC0 = decltype(has_c0)::value;
                     for (int c = 0; c < cols; c += 4, off2 += 4 * step) {
-                        double c0v[4];
+                        long long ac[4];
+                        int e[4];
+                        double c0v[4] = {}, r4[4];
 #pragma unroll
-                        for (int u = 0; u < 4; ++u) c0v[u] = c + u < cols ? C0d[off2 + u * step] : 0.0;
+                        for (int u = 0; u < 4; ++u) {
+                            ac[u] = sacc[(c + u) * 256 + et];  // columns past n: zeros
+                            e[u] = er + se[c + u];
+                            if (kC0 && c + u < cols) c0v[u] = C0d[off2 + u * step];
+                        }
+                        finish_four<kC0>(ac, e, plan.s0, neg, unit_scales, c0v, s_ab, s_c, r4);
 #pragma unroll
                         for (int u = 0; u < 4; ++u)
-                            if (c + u < cols)
-                                Cd[off2 + u * step] = finish_element<true>(sacc[(c + u) * 256 + et], er + se[c + u], plan.s0, neg,
-                                                                           unit_scales, c0v[u], s_ab, s_c);
+                            if (c + u < cols) Cd[off2 + u * step] = r4[u];
                     }
-                } else {
-#pragma unroll 4
-                    for (int c = 0; c < cols; ++c, off2 += step)
-                        Cd[off2] = finish_element<false>(sacc[c * 256 + et], er + se[c], plan.s0, neg, unit_scales, 0.0, s_ab, s_c);
-                }
+                };
+                if (C0d) finish(std::true_type{});
+                else finish(std::false_type{});
             }
         }
     }
