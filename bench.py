@@ -66,8 +66,8 @@ def workload(seed=SEED, n_points=N_POINTS, ridge=1.46):
 HERM_STAGE_DRAM_BYTES_PER_MATRIX_N121 = 33.0e6
 
 
-HERM_STAGE_KERNELS = ("eigensolve stage: herm_panel_batch_kernel (blocked tridiagonalisation, FP64) + tensor-core "
-                      "trailing updates + herm_ql_kernel + herm_apply_real_kernel (QL, FP64; its rotations on a real "
+HERM_STAGE_KERNELS = ("eigensolve stage: herm_panel_fixed_kernel (blocked tridiagonalisation, fixed point) + tensor-core "
+                      "trailing updates + herm_ql_fixed_kernel + herm_apply_real_kernel (QL and its rotations on a real "
                       "identity in 64-bit fixed point on the integer pipes) + tensor-core back-transformation")
 
 
@@ -398,7 +398,7 @@ def run_ours(args):
                 "clocks": clocks,
                 "e2e": {"value": e2e_value, "unit": "solves/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h},
                 "gpu_launches": launches,
-                "roofline": {"bound": "fp64", "kernel": (HERM_STAGE_KERNELS if herm else "eig_batch_kernel"),
+                "roofline": {"bound": "fp64", "kernel": (HERM_STAGE_KERNELS if herm else "fix_schur_kernel"),
                              "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
                              "traffic": (HERM_STAGE_DRAM_BYTES_PER_MATRIX_N121 * P
                                          if herm and n == 121 and HERM_STAGE_DRAM_BYTES_PER_MATRIX_N121 else None),
@@ -498,7 +498,7 @@ def lossy_rate(eng, torch, est, flush, args, peak):
             err = max(err, float(np.max(np.abs(host[key][pol * P + idx] - ref[key]))))
     return {"value": value, "unit": "solves/s", "steps": args.lossy_steps, "ms_per_step": total / args.lossy_steps,
             "gpu_launches": launches, "ridge_index": [LOSSY_RIDGE.real, LOSSY_RIDGE.imag],
-            "eigensolver": "general: Hessenberg reduction + shifted complex QR + back substitution (eig_batch_kernel)",
+            "eigensolver": "general: Hessenberg reduction + shifted complex QR + back substitution (fix_schur_kernel, 64-bit fixed point)",
             "eig_ms_per_step": eig_ms, "eig_busy_ms_per_step": eig_busy,
             "eig_roofline": {"achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                              "frac": achieved / peak if achieved else None, "flops_model": "105 n^3 per matrix"},
@@ -632,7 +632,7 @@ def run_secondary(args):
     # launch cost a little)
     eng.set_kernel_timing(True)
     step()
-    roof_kernel, flops_model = "eig_batch_kernel", "general QR: 105 n^3 per matrix"
+    roof_kernel, flops_model = "fix_schur_kernel", "general QR: 105 n^3 per matrix"
     if herm_model and not os.environ.get("RCWA_GB300_HERMITIAN", "").startswith("0"):
         # lossless layers: the Hermitian eigensolver; the model counts its matrices only (the few conical
         # Schur-basis eigensolves of order 2N inside the same timer are not counted)
