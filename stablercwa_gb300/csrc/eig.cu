@@ -296,14 +296,17 @@ void launch_eig_herm(cudaStream_t st, int n, int batch, const zc* a, long long a
         if (autotune_wanted(1, n, batch)) autotune_eig(st, 1, n, batch, a, a_stride, nullptr);
         group = tuned_eig_form(1, n, batch);
     }
-    // fixed point (eig_fixed.cuh) with the default settings: the QL iteration always, the reduction where no FP64
-    // form is forced or recorded and the batch is small (herm_fixed_reduce_wanted)
-    const bool fixed = eps == DBL_EPSILON && max_iter >= 30 && eig_fixed_enabled();
-    const bool fixed_reduce = fixed && group == 0 && herm_fixed_reduce_wanted(n, batch);
-    if (group <= 0) group = eig_default_group(n, batch);
-    TimedLaunch timed(TK_EIG, st);
     const size_t ysm = (size_t)n * kHermRows * sizeof(double);
     const bool real_form = ysm + kHermApplyStaticSmem <= 227 * 1024;
+    // fixed point (eig_fixed.cuh) with the default settings: the QL iteration always, the reduction where no FP64
+    // form is forced or recorded and the batch is small (herm_fixed_reduce_wanted). Divide and conquer takes d, e and Q
+    // of every matrix as they come, so it follows a reduction that writes them for every matrix: the fixed-point one
+    // leaves those of a matrix that it declines (zero, not finite, far out of scale) unwritten.
+    const bool fixed = eps == DBL_EPSILON && max_iter >= 30 && eig_fixed_enabled();
+    const bool dc = real_form && herm_dc_wanted(group > 0 ? group : eig_default_group(n, batch));
+    const bool fixed_reduce = fixed && !dc && group == 0 && herm_fixed_reduce_wanted(n, batch);
+    if (group <= 0) group = eig_default_group(n, batch);
+    TimedLaunch timed(TK_EIG, st);
     zc* q = v;
     double* y = nullptr;
     const bool blocked = !fixed_reduce && real_form && herm_blocked_wanted(n, group);
@@ -325,7 +328,6 @@ void launch_eig_herm(cudaStream_t st, int n, int batch, const zc* a, long long a
     } else {
         herm_reduce_dispatch(st, n, batch, a, a_stride, q, ws, group);
     }
-    const bool dc = real_form && herm_dc_wanted(group);
     const size_t qsm = (size_t)2 * n * kHermQlThreads * sizeof(double);
     if (dc) {
         switch (group) {
