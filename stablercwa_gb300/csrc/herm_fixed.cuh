@@ -17,6 +17,8 @@
 // at 2^-53 of themselves, every partial sum again. The scalars of a column, v, w and T stay in FP64.
 #pragma once
 
+#include <climits>
+
 #include "eig_fixed.cuh"
 
 namespace rcwa_gb300 {
@@ -206,6 +208,7 @@ __device__ void herm_panel_fixed(int n, int k0, int ex, zc* __restrict__ ws, zc*
         grp.sync();  // v is complete
         if (is_zero(tau)) {  // H_j = I: w = 0 and T's column is zero (both already)
             if (g == 0) wex[i] = 0;
+            grp.sync();  // the next column's updates read it
             continue;
         }
         // y = A0 v over the trailing block, owned rows, up to four a pass
