@@ -171,6 +171,9 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
 // A row of A or column of B holding a non-finite entry gets this exponent: its digits come out zero and
 // the epilogue writes NaN for every element of C it touches (any such product is non-finite in FP64 too).
 constexpr int kNonFinite = 1 << 20;
+// and a zero row or column this one, far below every other: the product's unit is then below any C0, which is kept as it
+// is. (With exponent 0 C0 was rounded to 2^-55, whatever its size: a solve lost the rows of a small diagonal block.)
+constexpr int kZeroLine = -(1 << 18);
 
 // The split kernels use no FP64 arithmetic: the FP64 pipe of this GPU runs 1/32 of the FP32 rate, and
 // conversions between FP64 and 64-bit integers run there too. Magnitudes are compared as the bit patterns
@@ -183,10 +186,10 @@ __device__ __forceinline__ unsigned long long mag_bits(double x) {
 }
 
 // the scale exponent of a row or column from its largest magnitude's bits: max = f 2^e with f in [0.5, 1);
-// kNonFinite when the row or column holds a non-finite entry, 0 when it is zero
+// kNonFinite when the row or column holds a non-finite entry, kZeroLine when it is zero
 __device__ __forceinline__ int scale_exponent(unsigned long long mb) {
     if (mb >= kMagInf) return kNonFinite;
-    if (mb == 0) return 0;
+    if (mb == 0) return kZeroLine;
     const int be = (int)(mb >> 52);
     if (be == 0) {  // a subnormal maximum (the FP64 path: rare)
         int e;
