@@ -386,7 +386,12 @@ int rcwa_gpu_kernel_busy(rcwa_gpu_ctx* ctx, const char* kind, double* millisecon
 /* Batched general complex eigensolver, CORTH + COMQR2 (include/stablercwa/eig_qr.hpp:1008-1124):
  * the engine behind Options::custom_eig (include/stablercwa/rcwa1d.hpp:122-124). a holds batch
  * n x n matrices; values[batch*n], vectors[batch*n*n] (2-norm normalised columns), info[batch]
- * (0 or the 1-based index of the eigenvalue that hit max_iter), sweeps[batch] (may be NULL). */
+ * (0 or the 1-based index of the eigenvalue that hit max_iter), sweeps[batch] (may be NULL).
+ * rcwa_gpu_eig_batch, and rcwa_gpu_eig_batch_dev with d_sweeps, iterate in FP64. Without d_sweeps, with eps = 2^-52,
+ * max_iter >= 30 and no form forced, orders 24 to 440 are solved in 64-bit fixed point: residuals as in FP64 or smaller, every
+ * eigenvalue to about 2^-58 of ||A||_2, however small it is itself. Matrices whose small eigenvalues FP64 would keep
+ * relative to themselves go to the FP64 kernels: upper triangular ones, and those whose last row or column is below 2^-7
+ * of the largest (graded downwards, or with a separate small block last). */
 int rcwa_gpu_eig_batch(rcwa_gpu_ctx* ctx, int n, int batch, const rcwa_complex* a, double eps, int max_iter,
                        rcwa_complex* values, rcwa_complex* vectors, int* info, int* sweeps);
 int rcwa_gpu_eig_batch_dev(rcwa_gpu_ctx* ctx, int n, int batch, const rcwa_complex* d_a, double eps,
@@ -398,14 +403,18 @@ int rcwa_gpu_eig_batch_dev(rcwa_gpu_ctx* ctx, int n, int batch, const rcwa_compl
  * accumulated). It solves the Hermitian part (a + a^H) / 2 of each of the batch n x n matrices in a (a itself
  * when a is Hermitian). values[batch*n] are real (imaginary parts 0) in the order the QL iteration leaves
  * them, not sorted; vectors[batch*n*n] have orthonormal columns; info[batch] is 0 or the 1-based index of
- * the eigenvalue that hit max_iter. eps and max_iter as in rcwa_gpu_eig_batch. */
+ * the eigenvalue that hit max_iter. eps and max_iter as in rcwa_gpu_eig_batch. With eps = 2^-52 and max_iter >= 30 the QL
+ * iteration (up to order 454) and parts of the reduction run in 64-bit fixed point, to about 2^-58 of ||A||_2 absolutely.
+ * Matrices with rows below 2^-7 of the largest take the FP64 kernels where practically nothing ties those rows to larger
+ * ones (diagonal matrices, separate blocks of different size) or the matrix is tridiagonal. RCWA_GB300_EIG_FIXED=0 keeps
+ * FP64 everywhere. */
 int rcwa_gpu_eig_hermitian_batch(rcwa_gpu_ctx* ctx, int n, int batch, const rcwa_complex* a, double eps, int max_iter,
                                  rcwa_complex* values, rcwa_complex* vectors, int* info);
 int rcwa_gpu_eig_hermitian_batch_dev(rcwa_gpu_ctx* ctx, int n, int batch, const rcwa_complex* d_a, double eps,
                                      int max_iter, rcwa_complex* d_values, rcwa_complex* d_vectors, int* d_info);
 
 /* Batched eigensolver that allocates nothing. No counterpart in the reference: it is the
- * rcwa_gpu_eig_batch_dev computation (same kernel and default lanes per matrix, so the same results) for callers
+ * rcwa_gpu_eig_batch_dev computation in FP64, as with sweep counts (same kernels and default lanes, so the same results), for callers
  * that may not allocate device memory -- a host whose own caching allocator holds the HBM, or a
  * latency-bound loop that cannot pay for an allocator call or the synchronisation a free implies.
  * The per-matrix workspace, 16 * (3n^2 + 4n + 8) bytes, comes from one fixed device array of

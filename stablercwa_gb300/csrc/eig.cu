@@ -190,12 +190,12 @@ void herm_panel_launch(cudaStream_t st, int n, int batch, int k0, const zc* a, l
 // trailing block's rank-2 nb update A -= V W^H + W V^H as two batched products (the tensor cores for
 // orders >= 32). vall receives the reflectors, mall the panels' T V^H.
 void herm_blocked_reduce(cudaStream_t st, int n, int batch, const zc* a, long long a_stride, zc* ws, zc* pan, zc* vall,
-                         zc* mall, int group, bool fixed) {
+                         zc* mall, int group, bool fixed, const int* other) {
     const int nb = kHermNb, P = herm_panel_count(n), pnb = P * nb;
     const long long ws_stride = eig_workspace_elems(n), pan_stride = herm_panel_elems(n);
     for (int b = 0; b < P; ++b) {
         const int k0 = b * nb;
-        if (fixed) launch_herm_panel_fixed(st, n, batch, k0, a, a_stride, ws, pan, vall, mall, pnb, group);
+        if (fixed) launch_herm_panel_fixed(st, n, batch, k0, a, a_stride, ws, pan, vall, mall, pnb, group, other);
         else switch (group) {
             case 4: herm_panel_launch<4>(st, n, batch, k0, a, a_stride, ws, pan, vall, mall, pnb); break;
             case 8: herm_panel_launch<8>(st, n, batch, k0, a, a_stride, ws, pan, vall, mall, pnb); break;
@@ -311,19 +311,24 @@ void launch_eig_herm(cudaStream_t st, int n, int batch, const zc* a, long long a
     double* y = nullptr;
     const bool blocked = !fixed_reduce && real_form && herm_blocked_wanted(n, group);
     zc *pan = nullptr, *mall = nullptr, *u = nullptr;
-    int* status = nullptr;  // matrices the fixed-point reduction left to the fused kernel
+    // matrices that the fixed-point reduction left to the fused kernel (1), or that the FP64 reduction and QL iteration
+    // keep (kFixOther; fix_range_kernel says why)
+    int* status = nullptr;
     if (real_form) {
         RCWA_CUDA(cudaMallocAsync(&q, (size_t)batch * n * n * sizeof(zc), st));  // Q, or the reflectors when blocked
         RCWA_CUDA(cudaMallocAsync(&y, (size_t)batch * n * n * sizeof(double), st));
+    }
+    if (fixed && real_form) {
+        RCWA_CUDA(cudaMallocAsync(&status, (size_t)batch * sizeof(int), st));
+        if (!fixed_reduce) launch_herm_range(st, n, batch, a, a_stride, status);
     }
     if (blocked) {
         const size_t pnb = (size_t)herm_panel_count(n) * kHermNb;
         RCWA_CUDA(cudaMallocAsync(&pan, (size_t)batch * herm_panel_elems(n) * sizeof(zc), st));
         RCWA_CUDA(cudaMallocAsync(&mall, (size_t)batch * pnb * n * sizeof(zc), st));
         RCWA_CUDA(cudaMallocAsync(&u, (size_t)batch * kHermNb * n * sizeof(zc), st));
-        herm_blocked_reduce(st, n, batch, a, a_stride, ws, pan, q, mall, group, fixed);
+        herm_blocked_reduce(st, n, batch, a, a_stride, ws, pan, q, mall, group, fixed, status);
     } else if (fixed_reduce) {
-        RCWA_CUDA(cudaMallocAsync(&status, (size_t)batch * sizeof(int), st));
         launch_herm_reduce_fixed(st, n, batch, a, a_stride, q, ws, status);
     } else {
         herm_reduce_dispatch(st, n, batch, a, a_stride, q, ws, group);
@@ -336,13 +341,20 @@ void launch_eig_herm(cudaStream_t st, int n, int batch, const zc* a, long long a
             case 16: herm_dc_launch<16>(st, n, batch, ws, y, w, info, eps, max_iter); break;
             default: herm_dc_launch<32>(st, n, batch, ws, y, w, info, eps, max_iter); break;
         }
-    } else if (fixed && real_form && qsm <= 227 * 1024) {
-        launch_herm_ql_fixed(st, n, batch, w, info, ws, status);
     } else if (qsm <= 227 * 1024) {
-        if (qsm > 48 * 1024) ensure_smem_optin(reinterpret_cast<const void*>(herm_ql_kernel<true, true>), (int)qsm);
-        // the real form's log is fixed point (herm_apply_real_kernel); the shared-memory form implies it
-        herm_ql_kernel<true, true><<<(unsigned)((batch + kHermQlThreads - 1) / kHermQlThreads), kHermQlThreads, qsm, st>>>(
-            n, batch, w, info, ws, eps, max_iter, rotation_counter());
+        if (fixed && real_form) {
+            launch_herm_ql_fixed(st, n, batch, w, info, ws, status);
+            // those that keep FP64: seldom any, so d and e stay in the workspace (with 16 n bytes of shared memory a matrix
+            // the launch waits for room beside the other polarisation's kernels)
+            if (!fixed_reduce)
+                herm_ql_kernel<false, true><<<(unsigned)((batch + 127) / 128), 128, 0, st>>>(n, batch, w, info, ws, eps, max_iter,
+                                                                                             rotation_counter(), status, kFixOther);
+        } else {
+            if (qsm > 48 * 1024) ensure_smem_optin(reinterpret_cast<const void*>(herm_ql_kernel<true, true>), (int)qsm);
+            // the real form's log is fixed point (herm_apply_real_kernel); the shared-memory form implies it
+            herm_ql_kernel<true, true><<<(unsigned)((batch + kHermQlThreads - 1) / kHermQlThreads), kHermQlThreads, qsm, st>>>(
+                n, batch, w, info, ws, eps, max_iter, rotation_counter());
+        }
     } else if (real_form) {
         herm_ql_kernel<false, true><<<(unsigned)((batch + 127) / 128), 128, 0, st>>>(n, batch, w, info, ws, eps,
                                                                                      max_iter, rotation_counter());
@@ -370,7 +382,7 @@ void launch_eig_herm(cudaStream_t st, int n, int batch, const zc* a, long long a
         } else {
             launch_zdgemm(st, n, n, n, batch, q, n, (long long)n * n, y, n, (long long)n * n, v, n, (long long)n * n, only, 1);
         }
-        launch_count() += dc ? 3 : 5;  // the overflow flags, the fused redo, and the reduction or r2c; QL and rotations
+        launch_count() += dc ? 3 : fixed && !fixed_reduce ? 6 : 5;  // the overflow flags, the fused redo, and the reduction or r2c; QL and rotations
     } else {
         herm_apply_kernel<<<(unsigned)(((long long)batch * n + 127) / 128), 128, 0, st>>>(n, batch, v, ws, info);
         RCWA_CUDA(cudaGetLastError());

@@ -1065,14 +1065,17 @@ __device__ inline int4 herm_fixed_entry(double c, double s) {
 // rotation chain is the whole cost, so with SMEM the thread's d and e live in shared memory (kHermQlThreads
 // threads per CTA, 16 n bytes each) rather than in the workspace, whose loads would sit on the chain.
 // FIXED logs each rotation as herm_fixed_entry(c, s), the fixed-point form herm_apply_real_kernel applies
-// on the integer pipes; else as the doubles (c, s) herm_apply_kernel applies to the complex Q.
+// on the integer pipes; else as the doubles (c, s) herm_apply_kernel applies to the complex Q. only: matrices whose
+// entry is only_value (the others are another kernel's).
 constexpr int kHermQlThreads = 32;
+constexpr int kFixOther = 2;  // status of a matrix that the FP64 reduction and iteration keep (eig_fixed.cuh)
 template <bool SMEM, bool FIXED>
 __global__ void __launch_bounds__(128) herm_ql_kernel(int n, int batch, zc* __restrict__ w, int* __restrict__ info,
                                                       zc* __restrict__ ws, double eps, int max_iter,
-                                                      unsigned long long* rotations) {
+                                                      unsigned long long* rotations, const int* __restrict__ only = nullptr,
+                                                      int only_value = 0) {
     const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (gid >= batch) return;
+    if (gid >= batch || (only && only[gid] != only_value)) return;
     zc* base = ws + gid * eig_workspace_elems(n);
     // d and e: this thread's column of the CTA's shared array (SMEM), else the H block of the workspace
     double* d;

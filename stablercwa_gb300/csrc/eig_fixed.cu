@@ -42,6 +42,16 @@ void fix_apply(cudaStream_t st, int n, int batch, zc* z, long long z_stride, con
         fix_apply_rows<32>(st, n, batch, z, z_stride, log, log_stride, table, head, status);
 }
 
+template <bool Herm>
+void fix_range(cudaStream_t st, int n, int batch, const zc* a, long long a_stride, int* status, int other) {
+    // Small CTAs where there are many matrices: they find room beside another stream's kernels (the mirror sweep, 4096 matrices
+    // of order 121 a stream, 363.8 ms without this kernel: 365.1 with 64 threads, 365.8 with 128, 366.0 with 512).
+    const int threads = batch >= 608 ? 64 : kFixRangeThreads;
+    fix_range_kernel<Herm><<<(unsigned)batch, threads, fix_range_smem(n), st>>>(n, batch, a, a_stride, status, other);
+    ++launch_count();
+    RCWA_CUDA(cudaGetLastError());
+}
+
 }  // namespace
 
 // RCWA_GB300_EIG_FIXED=0 keeps the FP64 iterations
@@ -70,8 +80,10 @@ void launch_eig_fixed(cudaStream_t st, int n, int batch, const zc* a, long long 
     const int chunk = (int)std::max(1LL, std::min<long long>(std::min(batch, std::max(kFixPassMin, (batch + 1) / 2)),
                                                              kFixLogBytes / eig_fixed_bytes(n)));
     int4 *log = nullptr, *table = nullptr;
-    int *head = nullptr, *status = nullptr;
+    int *head = nullptr, *status = nullptr, *other = nullptr;
     unsigned long long* tn = nullptr;
+    RCWA_CUDA(cudaMallocAsync(&other, (size_t)batch * sizeof(int), st));
+    fix_range<false>(st, n, batch, a, a_stride, other, 1);
     RCWA_CUDA(cudaMallocAsync(&log, (size_t)chunk * 2 * fix_log_capacity(n) * sizeof(int4), st));
     RCWA_CUDA(cudaMallocAsync(&table, (size_t)chunk * fix_table_capacity(n) * sizeof(int4), st));
     RCWA_CUDA(cudaMallocAsync(&head, (size_t)chunk * 2 * sizeof(int), st));
@@ -84,7 +96,7 @@ void launch_eig_fixed(cudaStream_t st, int n, int batch, const zc* a, long long 
         zc *z1 = wsc + nn, *z2 = wsc + 2 * nn;  // Z; X
         lz* h = reinterpret_cast<lz*>(wsc);
         fix_schur_kernel<false><<<(unsigned)cb, 32 * warps, schur_smem, st>>>(n, cb, ac, a_stride, wc, h, wst, log, 2 * fix_log_capacity(n), table, head, status,
-                                                                       done + b0, info + b0);
+                                                                       done + b0, info + b0, other + b0);
         RCWA_CUDA(cudaGetLastError());
         fix_apply(st, n, cb, z1, wst, log, 2 * fix_log_capacity(n), table, head, status);
         zc* t = t_out ? t_out + (long long)b0 * nn : vc;
@@ -104,27 +116,35 @@ void launch_eig_fixed(cudaStream_t st, int n, int batch, const zc* a, long long 
         RCWA_CUDA(cudaGetLastError());
         launch_count() += 2;
     }
-    for (void* p : {(void*)log, (void*)table, (void*)head, (void*)status, (void*)tn}) RCWA_CUDA(cudaFreeAsync(p, st));
+    for (void* p : {(void*)log, (void*)table, (void*)head, (void*)status, (void*)other, (void*)tn}) RCWA_CUDA(cudaFreeAsync(p, st));
+}
+
+// status[b] = kFixOther for a matrix that the FP64 reduction and QL iteration keep, else 0
+void launch_herm_range(cudaStream_t st, int n, int batch, const zc* a, long long a_stride, int* status) {
+    fix_range<true>(st, n, batch, a, a_stride, status, kFixOther);
 }
 
 // The Hermitian solver's reduction: d and e into ws (where the QL kernel reads them) and Q (n x n, contiguous);
-// status[b] = 1 for a matrix left to the FP64 kernels.
+// status[b] = 1 for a matrix left to the fused FP64 kernel.
 void launch_herm_reduce_fixed(cudaStream_t st, int n, int batch, const zc* a, long long a_stride, zc* q, zc* ws, int* status) {
     const long long nn = (long long)n * n, wst = 3 * nn + 4LL * n + 8, log_stride = 2 * fix_reduce_capacity(n);
     const int warps = fix_warps(n);
     const size_t schur_smem = fix_schur_smem(n, warps);
     ensure_smem_optin(reinterpret_cast<const void*>(fix_schur_kernel<true>), (int)schur_smem);
     int4* log = nullptr;
-    int* head = nullptr;
+    int *head = nullptr, *other = nullptr;
     RCWA_CUDA(cudaMallocAsync(&log, (size_t)batch * log_stride * sizeof(int4), st));
     RCWA_CUDA(cudaMallocAsync(&head, (size_t)batch * 2 * sizeof(int), st));
+    RCWA_CUDA(cudaMallocAsync(&other, (size_t)batch * sizeof(int), st));
+    fix_range<true>(st, n, batch, a, a_stride, other, 1);
     fix_schur_kernel<true><<<(unsigned)batch, 32 * warps, schur_smem, st>>>(n, batch, a, a_stride, nullptr, reinterpret_cast<lz*>(ws), wst,
-                                                                            log, log_stride, nullptr, head, status, nullptr, nullptr);
+                                                                            log, log_stride, nullptr, head, status, nullptr, nullptr, other);
     RCWA_CUDA(cudaGetLastError());
     fix_apply(st, n, batch, q, nn, log, log_stride, nullptr, head, status);
     launch_count() += 2;
     RCWA_CUDA(cudaFreeAsync(log, st));
     RCWA_CUDA(cudaFreeAsync(head, st));
+    RCWA_CUDA(cudaFreeAsync(other, st));
 }
 
 void launch_herm_ql_fixed(cudaStream_t st, int n, int batch, zc* w, int* info, zc* ws, const int* status) {
@@ -144,19 +164,19 @@ void launch_herm_ql_fixed(cudaStream_t st, int n, int batch, zc* w, int* info, z
 namespace {
 template <int G>
 void panel_launch(cudaStream_t st, int n, int batch, int k0, const zc* a, long long a_stride, zc* ws, zc* pan, zc* vall, zc* mall,
-                  int pnb) {
+                  int pnb, const int* other) {
     const unsigned blocks = (unsigned)(((long long)batch * G + 127) / 128);
-    herm_panel_fixed_kernel<G><<<blocks, 128, 0, st>>>(n, batch, k0, a, a_stride, ws, pan, vall, mall, pnb);
+    herm_panel_fixed_kernel<G><<<blocks, 128, 0, st>>>(n, batch, k0, a, a_stride, ws, pan, vall, mall, pnb, other);
 }
 }  // namespace
 
 void launch_herm_panel_fixed(cudaStream_t st, int n, int batch, int k0, const zc* a, long long a_stride, zc* ws, zc* pan, zc* vall,
-                             zc* mall, int pnb, int group) {
+                             zc* mall, int pnb, int group, const int* other) {
     switch (group) {
-        case 4: panel_launch<4>(st, n, batch, k0, a, a_stride, ws, pan, vall, mall, pnb); break;
-        case 8: panel_launch<8>(st, n, batch, k0, a, a_stride, ws, pan, vall, mall, pnb); break;
-        case 16: panel_launch<16>(st, n, batch, k0, a, a_stride, ws, pan, vall, mall, pnb); break;
-        case 32: panel_launch<32>(st, n, batch, k0, a, a_stride, ws, pan, vall, mall, pnb); break;
+        case 4: panel_launch<4>(st, n, batch, k0, a, a_stride, ws, pan, vall, mall, pnb, other); break;
+        case 8: panel_launch<8>(st, n, batch, k0, a, a_stride, ws, pan, vall, mall, pnb, other); break;
+        case 16: panel_launch<16>(st, n, batch, k0, a, a_stride, ws, pan, vall, mall, pnb, other); break;
+        case 32: panel_launch<32>(st, n, batch, k0, a, a_stride, ws, pan, vall, mall, pnb, other); break;
         default: throw EngineError{RCWA_EINVAL, "eig: the blocked Hermitian reduction takes 4, 8, 16 or 32 lanes"};
     }
     ++launch_count();

@@ -286,6 +286,125 @@ __device__ __forceinline__ lz fix_left_block(int n, lz* H, lz* tile, const int4*
     return y;
 }
 
+// ---- which matrices the fixed-point kernels may take
+//
+// One unit of 2^-59 N or less is lost wherever an entry is held: a row of size m keeps 2^-59 N / m of itself, however small
+// m is. FP64 loses more where its reflectors or shifts mix such a row with those of size N, as on a layer matrix
+// Kx^2 - [[eps]], whose centre is 2^-16 of N and tied to the rest by the profile's harmonics; where they do not it keeps
+// 2^-53 of the row, and such matrices stay with the FP64 kernels:
+//   - general solver: upper triangular matrices, and those whose last row or column is 2^-7 below the largest (graded
+//     downwards, or a small block last: deflated before a large shift has passed over them). A layer's last order is one
+//     of its largest (2^-4 of it at grazing incidence on a wide period).
+//   - Hermitian solver: rows 2^-7 below the largest that nothing ties to larger ones (diagonal matrices, separate blocks),
+//     in which the entries towards rows 2^3 larger are below 2^-40 of the row, or, 2^-14 below the largest, those
+//     towards rows 2^7 larger below 2^-16; and tridiagonal matrices with a row 2^-7 below the largest. The centre rows of layers,
+//     contrasts of a few percent among them, are tied by 2^-12 and more, for periods of 0.1 to 10 wavelengths.
+// Largest relative error of an eigenvalue at order 30 against 60 digits, FP64 / fixed point: diag(1 .. 1e-20) 0 / 1; a
+// block of 1e-4 of the other 3e-15 / 3e-12 (last, general), 2e-14 / 1e-12 (Hermitian); rows and columns graded downwards
+// over 1e-5 each, general 4e-14 / 2e-7, over 1e-2.1 2e-14 / 4e-13; triangular 0 / 6e-6; tridiagonal graded over 1e-4
+// 8e-16 / 5e-11. What stays here: layers 2e-13 to 1e-11 / 2e-14 to 7e-13; graded upwards over 1e-5, general 4e-7 / 4e-8,
+// Hermitian 4e-7 / 9e-8; Hermitian graded downwards over 1e-5 8e-8 / 3e-8; a small block first, general, 8e-12 / 2e-12.
+// The magnitudes are the upper words of the larger component (a lower word alone counts as the smallest).
+constexpr int kFixRangeThreads = 512;
+constexpr int kFixRangeSmall = 7 << 20, kFixRangeFar = 14 << 20, kFixRangeTie = 16 << 20;
+constexpr int kFixRangeLarger = 3 << 20, kFixRangeUntied = 40 << 20;
+__host__ __device__ inline size_t fix_range_smem(int n) { return ((size_t)2 * n + 2) * sizeof(int); }
+
+__device__ __forceinline__ int fix_magnitude(const zc& z) {
+    const unsigned long long x = (unsigned long long)__double_as_longlong(z.re) << 1, y = (unsigned long long)__double_as_longlong(z.im) << 1;
+    const unsigned long long m = x > y ? x : y;
+    return m == 0 ? 0 : max((int)(m >> 33), 1);
+}
+
+// the largest of a warp's values (none negative)
+__device__ __forceinline__ int fix_warp_max(int v) {
+#ifdef __CUDA_ARCH__
+    return (int)__reduce_max_sync(0xffffffffu, (unsigned)v);
+#else
+    for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+#endif
+}
+
+__device__ __forceinline__ void fix_shared_max(int* p, int v) {
+#ifdef __CUDA_ARCH__
+    atomicMax(p, v);
+#else
+    *p = max(*p, v);
+#endif
+}
+
+// status[b]: `other` for a matrix that the FP64 kernels keep, else 0. A CTA per matrix, which it reads once (a warp takes
+// 32 rows of eight columns at a time, all loads in flight); then a warp for every small row or column. Latency bounds it
+// for one matrix (order 121: 11 us cold; with 128 threads, 32 rows and all columns a warp, 65), the memory for 4096 (0.18 ms).
+template <bool Herm>
+__global__ void __launch_bounds__(kFixRangeThreads) fix_range_kernel(int n, int batch, const zc* __restrict__ a_in, long long a_stride,
+                                                                     int* __restrict__ status, int other) {
+    RCWA_DYN_SMEM(int, fix_rg);
+    const long long gid = blockIdx.x;
+    if (gid >= batch) return;
+    const zc* A = a_in + gid * a_stride;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nthr = blockDim.x, nw = nthr >> 5;
+    int *rs = fix_rg, *cs = rs + n, *flags = cs + n;  // largest of each row and column; [0] beside the band, [1] the FP64 kernels'
+    for (int i = tid; i < 2 * n + 2; i += nthr) fix_rg[i] = 0;
+    __syncthreads();
+    bool outside = false;
+    const int chunks = (n + 31) / 32, items = chunks * ((n + 7) / 8);
+    for (int q = warp; q < items; q += nw) {
+        const int r = 32 * (q % chunks) + lane, c0 = 8 * (q / chunks);
+        const bool in = r < n;
+        const zc* a = A + (long long)c0 * n + (in ? r : n - 1);
+        int v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = fix_magnitude(a[(long long)min(u, n - 1 - c0) * n]);  // the last column again
+        int m = 0, col = 0;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int c = min(c0 + u, n - 1);
+            m = max(m, v[u]);
+            outside |= in && v[u] != 0 && (Herm ? c + 1 < r || r + 1 < c : c < r);
+            const int w = fix_warp_max(in ? v[u] : 0);
+            if (lane == u) col = w;
+        }
+        if (in) fix_shared_max(rs + r, m);
+        if (lane < 8) fix_shared_max(cs + min(c0 + lane, n - 1), col);
+    }
+    if (outside) flags[0] = 1;
+    __syncthreads();
+    int top = 0, high = 0;  // the largest, and 2^31 - 1 less the smallest that is not zero
+    for (int i = lane; i < n; i += 32) {
+        if (Herm && warp == 0) rs[i] = max(rs[i], cs[i]);
+        const int m = max(rs[i], cs[i]);
+        top = max(top, m);
+        if (m) high = max(high, 0x7fffffff - m);
+    }
+    top = fix_warp_max(top);
+    const int low = 0x7fffffff - fix_warp_max(high);
+    if (Herm) __syncthreads();
+    bool keep = false;
+    if (top != 0 && top < 0x7ff00000) {  // zero and non-finite matrices are the solvers' own to leave
+        if (!Herm) {
+            int last = n - 1;
+            while (min(rs[last], cs[last]) == 0 && last > 0) --last;
+            keep = !flags[0] || min(rs[last], cs[last]) + kFixRangeSmall <= top;
+        } else if (low + kFixRangeSmall <= top) {
+            keep = !flags[0];
+            for (int i = warp; i < n; i += nw) {
+                const int m = rs[i];
+                if (m == 0 || m + kFixRangeSmall > top) continue;
+                const bool far = m + kFixRangeFar <= top;
+                int tie = 0;
+                for (int k = lane; k < n; k += 32)
+                    if (rs[k] >= m + (far ? kFixRangeSmall : kFixRangeLarger)) tie = max(tie, max(fix_magnitude(A[(long long)k * n + i]), fix_magnitude(A[(long long)i * n + k])));
+                keep |= fix_warp_max(tie) + (far ? kFixRangeTie : kFixRangeUntied) <= m;
+            }
+        }
+    }
+    if (keep) flags[1] = 1;
+    __syncthreads();
+    if (tid == 0) status[gid] = flags[1] ? other : 0;
+}
+
 constexpr int kFixBatch = 6;  // columns whose entries a row's lane holds at once, and as many on their way
 
 // Schur reduction of one matrix; with Herm only step 1, on the Hermitian part (A + A^H) / 2: the reduced matrix is
@@ -297,10 +416,17 @@ template <bool Herm>
 __global__ void fix_schur_kernel(int n, int batch, const zc* __restrict__ a_in, long long a_stride, zc* __restrict__ w_out,
                                         lz* __restrict__ h_ws, long long h_stride, int4* __restrict__ log_all, long long log_stride,
                                         int4* __restrict__ table_all, int* __restrict__ head, int* __restrict__ status,
-                                        int* __restrict__ done, int* __restrict__ info) {
+                                        int* __restrict__ done, int* __restrict__ info, const int* __restrict__ other = nullptr) {
     RCWA_DYN_SMEM(lz, fix_sm);
     const long long gid = blockIdx.x;
     if (gid >= batch) return;
+    if (other && other[gid]) {
+        if (threadIdx.x == 0) {
+            status[gid] = 1;
+            if (!Herm) done[gid] = 0;
+        }
+        return;
+    }
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nthr = blockDim.x, nw = nthr >> 5;
     lz* tiles = fix_sm;
     lz* tile = tiles + (long long)warp * kFixTile;
@@ -999,8 +1125,8 @@ static __global__ void __launch_bounds__(128) fix_unit_columns_kernel(int n, int
 // as FP64's, whose rounding follows the entries; now they are closer (reflection amplitudes of order-301 layers, mean
 // relative error: FP64 5.4e-12, whole units 1.4e-11, these 2.2e-12). What it does
 // not finish (non-finite or zero matrices, scales whose powers of two are not normal doubles, 30 sweeps without a
-// deflation) is flagged as a full log is, for the fused FP64 kernel. status, if given: matrices whose reduction left
-// them to that kernel already.
+// deflation) is flagged as a full log is, for the fused FP64 kernel. status, if given: 1 for matrices whose reduction
+// left them to that kernel already, kFixOther for those of herm_ql_kernel.
 constexpr int kFixQlBits = 59;
 constexpr int kFixQlExtra = 3;  // bits below one unit of d and e in memory
 
@@ -1054,7 +1180,8 @@ static __global__ void __launch_bounds__(kHermQlThreads) herm_ql_fixed_kernel(in
     // the scale
     float big = 0.0f;
     int e2 = 0;
-    bool usable = !(status && status[gid]);
+    const int set = status ? status[gid] : 0;
+    bool usable = set == 0;
     if (usable) {
         int top = 0;
         for (int k = 0; k < 2 * n; ++k) top = max(top, (int)((__double_as_longlong(src[k]) >> 52) & 0x7FF));
@@ -1070,9 +1197,11 @@ static __global__ void __launch_bounds__(kHermQlThreads) herm_ql_fixed_kernel(in
             e2 = ((__float_as_int(big * 1.001f) >> 23) & 0xff) - 127 + 1 + (top - 1023) - kFixQlBits;
         }
     }
-    tail[0] = 0;
-    tail[1] = !usable;
-    info[gid] = 0;
+    if (set != kFixOther) {
+        tail[0] = 0;
+        tail[1] = !usable;
+        info[gid] = 0;
+    }
     if (!usable) return;
     for (int k = 0; k < n; ++k) {
         d[k * sd] = fix_from_double(src[k], e2 - kFixQlExtra);

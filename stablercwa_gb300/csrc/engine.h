@@ -110,11 +110,13 @@ bool eig_fixed_possible(int n);
 long long eig_fixed_bytes(int n);
 void launch_eig_fixed(cudaStream_t st, int n, int batch, const zc* a, long long a_stride, zc* w, zc* v, int* info, zc* ws,
                       int* done, double eps, zc* t_out);
-// The Hermitian solver's pieces in fixed point: the reduction (d and e into ws, Q contiguous; status 1: left to the
-// FP64 kernels) and the QL iteration on d and e (status may be null).
+// The Hermitian solver's pieces in fixed point: which matrices they leave to the FP64 reduction and QL iteration (status
+// 2), the reduction (d and e into ws, Q contiguous; status 1: left to the fused FP64 kernel), its panels (other: matrices
+// for the FP64 panels) and the QL iteration on d and e.
+void launch_herm_range(cudaStream_t st, int n, int batch, const zc* a, long long a_stride, int* status);
 void launch_herm_reduce_fixed(cudaStream_t st, int n, int batch, const zc* a, long long a_stride, zc* q, zc* ws, int* status);
 void launch_herm_panel_fixed(cudaStream_t st, int n, int batch, int k0, const zc* a, long long a_stride, zc* ws, zc* pan, zc* vall,
-                             zc* mall, int pnb, int group);
+                             zc* mall, int pnb, int group, const int* other);
 void launch_herm_ql_fixed(cudaStream_t st, int n, int batch, zc* w, int* info, zc* ws, const int* status);
 bool eig_fixed_enabled();
 // The same product on the tensor cores (gemm_tc.cu: Ozaki-split bf16 tcgen05 products, FP64-accurate);

@@ -294,7 +294,7 @@ __device__ void herm_panel_fixed(int n, int k0, int ex, zc* __restrict__ ws, zc*
 }
 
 // The scale of the Hermitian part: 2^ex > N, or INT_MIN where N is zero, not finite or far from 1 (the FP64
-// panels take the matrix).
+// panels take the matrix, as they do where other[b] is set).
 template <int G>
 __device__ int herm_fix_scale(int n, const zc* __restrict__ A0) {
     const int g = threadIdx.x & (G - 1);
@@ -319,7 +319,7 @@ __device__ int herm_fix_scale(int n, const zc* __restrict__ A0) {
 template <int G>
 __global__ void __launch_bounds__(128) herm_panel_fixed_kernel(int n, int batch, int k0, const zc* __restrict__ a, long long a_stride,
                                                                zc* __restrict__ ws, zc* __restrict__ pan, zc* __restrict__ vall,
-                                                               zc* __restrict__ mall, int pnb) {
+                                                               zc* __restrict__ mall, int pnb, const int* __restrict__ other = nullptr) {
     const long long gid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / G;
     if (gid >= batch) return;
     zc* w = ws + gid * eig_workspace_elems(n);
@@ -332,7 +332,7 @@ __global__ void __launch_bounds__(128) herm_panel_fixed_kernel(int n, int batch,
     if (k0 == 0) {
         const int g = threadIdx.x & (G - 1);
         const Grp<G> grp(nullptr, nullptr);
-        ex = herm_fix_scale<G>(n, A0);
+        ex = other && other[gid] ? INT_MIN : herm_fix_scale<G>(n, A0);
         if (g == 0) *head = ex;
         if (ex != INT_MIN) {
             const double half = herm_fix_pow2(-ex - 1);
