@@ -42,12 +42,11 @@ void launch_eig(cudaStream_t st, int n, int batch, const zc* a, long long a_stri
     // FP64 kernels. The autotuner's table chooses among the FP64 forms, for the calls that take those.
     if (group == 0 && !skip && !sweeps && eps == DBL_EPSILON && max_iter >= 30 && eig_fixed_possible(n)) {
         TimedLaunch timed(TK_EIG, st);
-        int* done = nullptr;
-        RCWA_CUDA(cudaMallocAsync(&done, (size_t)batch * sizeof(int), st));
+        DeviceScratch mem(st);
+        int* done = mem.get<int>(batch);
         launch_eig_fixed(st, n, batch, a, a_stride, w, v, info, ws, done, eps, t_out);
         launch_eig_fp64(st, n, batch, a, a_stride, w, v, info, sweeps, ws, eps, max_iter, eig_default_group(n, batch), done, 1,
                         t_out);
-        RCWA_CUDA(cudaFreeAsync(done, st));
         return;
     }
     if (group == 0 && !skip && !t_out) {
@@ -307,6 +306,7 @@ void launch_eig_herm(cudaStream_t st, int n, int batch, const zc* a, long long a
     const bool fixed_reduce = fixed && !dc && group == 0 && herm_fixed_reduce_wanted(n, batch);
     if (group <= 0) group = eig_default_group(n, batch);
     TimedLaunch timed(TK_EIG, st);
+    DeviceScratch mem(st);
     zc* q = v;
     double* y = nullptr;
     const bool blocked = !fixed_reduce && real_form && herm_blocked_wanted(n, group);
@@ -315,18 +315,18 @@ void launch_eig_herm(cudaStream_t st, int n, int batch, const zc* a, long long a
     // keep (kFixOther; fix_range_kernel says why)
     int* status = nullptr;
     if (real_form) {
-        RCWA_CUDA(cudaMallocAsync(&q, (size_t)batch * n * n * sizeof(zc), st));  // Q, or the reflectors when blocked
-        RCWA_CUDA(cudaMallocAsync(&y, (size_t)batch * n * n * sizeof(double), st));
+        q = mem.get<zc>((size_t)batch * n * n);  // Q, or the reflectors when blocked
+        y = mem.get<double>((size_t)batch * n * n);
     }
     if (fixed && real_form) {
-        RCWA_CUDA(cudaMallocAsync(&status, (size_t)batch * sizeof(int), st));
+        status = mem.get<int>(batch);
         if (!fixed_reduce) launch_herm_range(st, n, batch, a, a_stride, status);
     }
     if (blocked) {
         const size_t pnb = (size_t)herm_panel_count(n) * kHermNb;
-        RCWA_CUDA(cudaMallocAsync(&pan, (size_t)batch * herm_panel_elems(n) * sizeof(zc), st));
-        RCWA_CUDA(cudaMallocAsync(&mall, (size_t)batch * pnb * n * sizeof(zc), st));
-        RCWA_CUDA(cudaMallocAsync(&u, (size_t)batch * kHermNb * n * sizeof(zc), st));
+        pan = mem.get<zc>((size_t)batch * herm_panel_elems(n));
+        mall = mem.get<zc>((size_t)batch * pnb * n);
+        u = mem.get<zc>((size_t)batch * kHermNb * n);
         herm_blocked_reduce(st, n, batch, a, a_stride, ws, pan, q, mall, group, fixed, status);
     } else if (fixed_reduce) {
         launch_herm_reduce_fixed(st, n, batch, a, a_stride, q, ws, status);
@@ -363,8 +363,7 @@ void launch_eig_herm(cudaStream_t st, int n, int batch, const zc* a, long long a
                                                                                       max_iter, rotation_counter());
     }
     RCWA_CUDA(cudaGetLastError());
-    int* only = nullptr;  // matrices whose log overflowed: the fused kernel, masked to them
-    RCWA_CUDA(cudaMallocAsync(&only, (size_t)batch * sizeof(int), st));
+    int* only = mem.get<int>(batch);  // matrices whose log overflowed: the fused kernel, masked to them
     herm_overflow_kernel<<<(unsigned)((batch + 127) / 128), 128, 0, st>>>(n, batch, ws, only);
     RCWA_CUDA(cudaGetLastError());
     if (real_form) {
@@ -389,17 +388,6 @@ void launch_eig_herm(cudaStream_t st, int n, int batch, const zc* a, long long a
         launch_count() += 4;
     }
     herm_fused_dispatch(st, n, batch, a, a_stride, w, v, info, ws, eps, max_iter, group, only);
-    RCWA_CUDA(cudaFreeAsync(only, st));
-    if (status) RCWA_CUDA(cudaFreeAsync(status, st));
-    if (real_form) {
-        RCWA_CUDA(cudaFreeAsync(q, st));
-        RCWA_CUDA(cudaFreeAsync(y, st));
-    }
-    if (blocked) {
-        RCWA_CUDA(cudaFreeAsync(pan, st));
-        RCWA_CUDA(cudaFreeAsync(mall, st));
-        RCWA_CUDA(cudaFreeAsync(u, st));
-    }
 }
 
 }  // namespace rcwa_gb300

@@ -79,16 +79,13 @@ void launch_eig_fixed(cudaStream_t st, int n, int batch, const zc* a, long long 
     if (back_smem > 48 * 1024) ensure_smem_optin(reinterpret_cast<const void*>(fix_backsub_kernel), (int)back_smem);
     const int chunk = (int)std::max(1LL, std::min<long long>(std::min(batch, std::max(kFixPassMin, (batch + 1) / 2)),
                                                              kFixLogBytes / eig_fixed_bytes(n)));
-    int4 *log = nullptr, *table = nullptr;
-    int *head = nullptr, *status = nullptr, *other = nullptr;
-    unsigned long long* tn = nullptr;
-    RCWA_CUDA(cudaMallocAsync(&other, (size_t)batch * sizeof(int), st));
+    DeviceScratch mem(st);
+    int* other = mem.get<int>(batch);
     fix_range<false>(st, n, batch, a, a_stride, other, 1);
-    RCWA_CUDA(cudaMallocAsync(&log, (size_t)chunk * 2 * fix_log_capacity(n) * sizeof(int4), st));
-    RCWA_CUDA(cudaMallocAsync(&table, (size_t)chunk * fix_table_capacity(n) * sizeof(int4), st));
-    RCWA_CUDA(cudaMallocAsync(&head, (size_t)chunk * 2 * sizeof(int), st));
-    RCWA_CUDA(cudaMallocAsync(&status, (size_t)chunk * sizeof(int), st));
-    RCWA_CUDA(cudaMallocAsync(&tn, (size_t)chunk * sizeof(unsigned long long), st));
+    int4* log = mem.get<int4>((size_t)chunk * 2 * fix_log_capacity(n));
+    int4* table = mem.get<int4>((size_t)chunk * fix_table_capacity(n));
+    int *head = mem.get<int>((size_t)chunk * 2), *status = mem.get<int>(chunk);
+    unsigned long long* tn = mem.get<unsigned long long>(chunk);
     for (int b0 = 0; b0 < batch; b0 += chunk) {
         const int cb = std::min(chunk, batch - b0);
         const zc* ac = a + (long long)b0 * a_stride;
@@ -116,7 +113,6 @@ void launch_eig_fixed(cudaStream_t st, int n, int batch, const zc* a, long long 
         RCWA_CUDA(cudaGetLastError());
         launch_count() += 2;
     }
-    for (void* p : {(void*)log, (void*)table, (void*)head, (void*)status, (void*)other, (void*)tn}) RCWA_CUDA(cudaFreeAsync(p, st));
 }
 
 // status[b] = kFixOther for a matrix that the FP64 reduction and QL iteration keep, else 0
@@ -131,20 +127,15 @@ void launch_herm_reduce_fixed(cudaStream_t st, int n, int batch, const zc* a, lo
     const int warps = fix_warps(n);
     const size_t schur_smem = fix_schur_smem(n, warps);
     ensure_smem_optin(reinterpret_cast<const void*>(fix_schur_kernel<true>), (int)schur_smem);
-    int4* log = nullptr;
-    int *head = nullptr, *other = nullptr;
-    RCWA_CUDA(cudaMallocAsync(&log, (size_t)batch * log_stride * sizeof(int4), st));
-    RCWA_CUDA(cudaMallocAsync(&head, (size_t)batch * 2 * sizeof(int), st));
-    RCWA_CUDA(cudaMallocAsync(&other, (size_t)batch * sizeof(int), st));
+    DeviceScratch mem(st);
+    int4* log = mem.get<int4>((size_t)batch * log_stride);
+    int *head = mem.get<int>((size_t)batch * 2), *other = mem.get<int>(batch);
     fix_range<true>(st, n, batch, a, a_stride, other, 1);
     fix_schur_kernel<true><<<(unsigned)batch, 32 * warps, schur_smem, st>>>(n, batch, a, a_stride, nullptr, reinterpret_cast<lz*>(ws), wst,
                                                                             log, log_stride, nullptr, head, status, nullptr, nullptr, other);
     RCWA_CUDA(cudaGetLastError());
     fix_apply(st, n, batch, q, nn, log, log_stride, nullptr, head, status);
     launch_count() += 2;
-    RCWA_CUDA(cudaFreeAsync(log, st));
-    RCWA_CUDA(cudaFreeAsync(head, st));
-    RCWA_CUDA(cudaFreeAsync(other, st));
 }
 
 void launch_herm_ql_fixed(cudaStream_t st, int n, int batch, zc* w, int* info, zc* ws, const int* status) {

@@ -925,13 +925,10 @@ void tc_product(cudaStream_t st, int m, int n, int k, int batch, const zc* A, in
     const int chunk = (int)std::max(1LL, std::min<long long>(batch, (1LL << 30) / per));
     int* err = error_flag();
 
-    uint16_t *pa = nullptr, *pb = nullptr;
-    int *dea = nullptr, *deb = nullptr;
     const int na = a_bcast ? 1 : chunk, nb = b_bcast ? 1 : chunk;
-    RCWA_CUDA(cudaMallocAsync(&pa, (size_t)a_bytes * na, st));
-    RCWA_CUDA(cudaMallocAsync(&pb, (size_t)b_bytes * nb, st));
-    RCWA_CUDA(cudaMallocAsync(&dea, sizeof(int) * (size_t)m * (a_bcast ? 1 : batch), st));
-    RCWA_CUDA(cudaMallocAsync(&deb, sizeof(int) * (size_t)n * (b_bcast ? 1 : batch), st));
+    DeviceScratch mem(st);
+    uint16_t *pa = mem.get<uint16_t>((size_t)a_bytes / 2 * na), *pb = mem.get<uint16_t>((size_t)b_bytes / 2 * nb);
+    int *dea = mem.get<int>((size_t)m * (a_bcast ? 1 : batch)), *deb = mem.get<int>((size_t)n * (b_bcast ? 1 : batch));
     const CUtensorMap map_a = plane_map(pa, 2LL * m, Kp, (long long)na * S);
     const CUtensorMap map_b = plane_map(pb, n, Kp, (long long)nb * S);
     if (a_bcast) {
@@ -958,10 +955,6 @@ void tc_product(cudaStream_t st, int m, int n, int k, int batch, const zc* A, in
         ++launch_count();
         RCWA_CUDA(cudaGetLastError());
     }
-    RCWA_CUDA(cudaFreeAsync(pa, st));
-    RCWA_CUDA(cudaFreeAsync(pb, st));
-    RCWA_CUDA(cudaFreeAsync(dea, st));
-    RCWA_CUDA(cudaFreeAsync(deb, st));
 }
 
 }  // namespace

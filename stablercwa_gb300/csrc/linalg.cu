@@ -147,12 +147,10 @@ void lu_solve_blocked(cudaStream_t st, int n, int nrhs, int batch, const zc* a, 
     // 5.9 against 5.2.
     const bool warp_panels = n <= 64 && batch >= 608;
     const int swap_stride = kSwapInts + (n > kPanelSmemRows ? n : 0);
-    int *sing_local = nullptr, *swaps = nullptr;
-    RCWA_CUDA(cudaMallocAsync(&sing_local, (size_t)batch * sizeof(int), st));
-    RCWA_CUDA(cudaMemsetAsync(sing_local, 0, (size_t)batch * sizeof(int), st));
-    zc* dinv = nullptr;
-    RCWA_CUDA(cudaMallocAsync(&dinv, (size_t)batch * n * sizeof(zc), st));
-    if (!warp_panels) RCWA_CUDA(cudaMallocAsync(&swaps, (size_t)batch * swap_stride * sizeof(int), st));
+    DeviceScratch mem(st);
+    int* sing_local = mem.zeros<int>(batch);
+    zc* dinv = mem.get<zc>((size_t)batch * n);
+    int* swaps = warp_panels ? nullptr : mem.get<int>((size_t)batch * swap_stride);
     const long long init = (long long)batch * n * (n + nrhs);
     lu_init_kernel<<<(unsigned)((init + 255) / 256), 256, 0, st>>>(n, nrhs, batch, a, a_stride, lu, lu_stride, rhs_kind, rhs,
                                                                    rhs_stride, x, x_stride, skip, skip_value);
@@ -221,9 +219,6 @@ void lu_solve_blocked(cudaStream_t st, int n, int nrhs, int batch, const zc* a, 
     lu_nan_fill_kernel<<<(unsigned)((xt + 255) / 256), 256, 0, st>>>(n, nrhs, batch, x, x_stride, sing_local, singular);
     ++launch_count();
     RCWA_CUDA(cudaGetLastError());
-    RCWA_CUDA(cudaFreeAsync(sing_local, st));
-    RCWA_CUDA(cudaFreeAsync(dinv, st));
-    if (swaps) RCWA_CUDA(cudaFreeAsync(swaps, st));
 }
 
 }  // namespace
