@@ -251,18 +251,21 @@ struct Job {
     Res2D r2;
 };
 
-// Device bytes one solve holds at its peak, from the engines' own working-set estimates: the
-// eigensolver workspace and the dense operators of the S-matrix recursion at the algebra order n.
+// Device bytes one solve holds at its peak: the eigensolver's workspace and rotation logs, the dense operators of the
+// S-matrix recursion at the algebra order n, and every grating's constant matrices (in TM 13 for a lossless one: the
+// Toeplitz matrices, their inverses and Cholesky factors, the pencil's parts; conical 12). Allocator high-water marks of one
+// request stay below it (three lossless TM gratings at M = 150: 86.7 MiB of 96; without the constants 42).
 double footprint_of(const Job& j) {
     const double z = 16.0;
     switch (j.req.kind) {
         case RCWA_REQ_1D: {
             const double n = 2.0 * j.req.M + 1;
-            return z * n * n * (3.0 * (j.s1.stack.n_layers + 1) + 12.0) + (1 << 20);
+            return z * n * n * (3.0 * (j.s1.stack.n_layers + 1) + 12.0 + (j.req.polarization == RCWA_TE ? 4.0 : 17.0) * j.s1.gratings) +
+                   (1 << 20);
         }
         case RCWA_REQ_CONICAL: {
             const double N = 2.0 * j.req.M + 1, n = 2 * N;
-            return z * (n * n * 16.0 + N * N * 12.0 * j.s1.gratings + n * 8.0 * (j.s1.stack.n_layers + 2)) +
+            return z * (n * n * 16.0 + N * N * 24.0 * j.s1.gratings + n * 8.0 * (j.s1.stack.n_layers + 2)) +
                    2.0 * z * (3 * N * N + 4 * N + 8) * std::max(1, j.s1.gratings) + (1 << 20);
         }
         default: {
