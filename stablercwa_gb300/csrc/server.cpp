@@ -30,6 +30,7 @@
 
 namespace rcwa_gb300 {
 void preload_eig_cluster_kernel();  // eig_cluster.cu
+long long eig_fixed_bytes(int n);   // eig_fixed.cu: the general eigensolver's rotation logs, a matrix
 }
 
 namespace {
@@ -270,7 +271,8 @@ double footprint_of(const Job& j) {
         }
         default: {
             const double N = (2.0 * j.req.M1 + 1) * (2.0 * j.req.M2 + 1), n = 2 * N;
-            return z * n * n * (5.0 * j.s2.patterned + 3.0 * (j.s2.stack.n_layers + 1) + 8.0) + (1 << 20);
+            return z * n * n * (5.0 * j.s2.patterned + 3.0 * (j.s2.stack.n_layers + 1) + 8.0) +
+                   (double)j.s2.patterned * (double)rcwa_gb300::eig_fixed_bytes((int)n) + (1 << 20);
         }
     }
 }
