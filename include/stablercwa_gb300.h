@@ -456,7 +456,7 @@ int rcwa_validate_solve_conical(const rcwa_stack1d* stack, const rcwa_point_coni
 int rcwa_validate_solve2d(const rcwa_stack2d* stack, const rcwa_point2d* points, int n_points, int M1, int M2,
                           int factorization, char* message, size_t size);
 
-/* No reference counterpart: the autotuner of the eigensolvers' kernel form. The batched eigensolvers run
+/* No reference counterpart: the autotuner of the FP64 eigensolvers' kernel form. These run
  * a matrix on G = 4..32 lanes of a warp, on a CTA of 64, 128 or 256 threads, or (general solver, order
  * >= 384) on a thread-block cluster; a fixed rule picks one unless a tuned form is recorded for the key
  * (solver, order, batch size rounded down to a power of two). rcwa_gpu_autotune_eig times every
@@ -466,8 +466,12 @@ int rcwa_validate_solve2d(const rcwa_stack2d* stack, const rcwa_point2d* points,
  * Hermitian solver (lossless layers) instead of the general one. rcwa_gpu_autotune_set records a form
  * directly (a table saved earlier); rcwa_gpu_autotune_table writes the table as text lines
  * "<general|hermitian> <order> <batch bucket> <form>" and returns its length. The table is process-wide.
- * RCWA_GB300_AUTOTUNE=0 makes the solves ignore it; =auto also tunes each new key (at least 64 matrices)
- * on the first call that meets it, on that call's own matrices. */
+ * The general solver's fixed-point form (rcwa_gpu_eig_batch_dev) does not look at it: recorded general forms serve calls
+ * with sweep counts, the static entry and orders outside 24 to 440. A form recorded for a Hermitian key takes the place
+ * of the fixed-point reduction that the rule has for small batches (n * batch <= 48000, and 360 matrices from order 64
+ * on), which is mostly the faster one; RCWA_GB300_AUTOTUNE=0 makes the solves ignore the table; =auto also tunes each new
+ * key (at least 64 matrices) that the rule leaves to the FP64 forms on the first call that meets it, on that call's own
+ * matrices. */
 int rcwa_gpu_autotune_eig(rcwa_gpu_ctx* ctx, int hermitian, int n, int batch, const rcwa_complex* d_a, int* form,
                           double* milliseconds);
 int rcwa_gpu_autotune_set(int hermitian, int n, int batch, int form);

@@ -1,15 +1,17 @@
-// autotune.cu -- the eigensolver's kernel form per (kind, order, batch size), picked by timing.
+// autotune.cu -- the FP64 eigensolvers' kernel form per (kind, order, batch size), picked by timing.
 //
-// The batched eigensolvers come in several forms: G = 4..32 lanes of a warp per matrix, a CTA of 64, 128
+// The batched FP64 eigensolvers come in several forms: G = 4..32 lanes of a warp per matrix, a CTA of 64, 128
 // or 256 threads per matrix, and (general solver, order >= 384) a thread-block cluster per matrix. Which
 // is fastest depends on the order, the batch and the device; the built-in rule (eig_default_group) is a
 // fixed heuristic. The tuner runs every applicable form on a batch of real matrices (each form twice, the
 // second run timed with CUDA events on the caller's stream), keeps only forms whose results agree with
 // the heuristic's form on convergence (info), and records the fastest for the key (solver kind, order,
-// batch size rounded down to a power of two). The launchers consult the table whenever no form is forced.
-// Tuning happens when asked (rcwa_gpu_autotune_eig) or, with RCWA_GB300_AUTOTUNE=auto, the first time a
-// launcher meets a key with at least 64 matrices, on that call's own matrices; RCWA_GB300_AUTOTUNE=0
-// ignores the table.
+// batch size rounded down to a power of two). The launchers consult the table whenever no form is forced and the
+// call takes those kernels: the general solver's fixed-point form (orders 24 to 440, no sweep counts asked for)
+// does not, and a form recorded for a Hermitian key replaces the fixed-point reduction that the built-in rule takes for
+// small batches. Tuning happens when asked (rcwa_gpu_autotune_eig) or, with RCWA_GB300_AUTOTUNE=auto, the first time a
+// launcher meets a key with at least 64 matrices that the built-in rule gives to these kernels, on that call's own
+// matrices; RCWA_GB300_AUTOTUNE=0 ignores the table.
 #include <cuda_runtime.h>
 
 #include <algorithm>

@@ -291,8 +291,14 @@ void herm_fused_dispatch(cudaStream_t st, int n, int batch, const zc* a, long lo
 void launch_eig_herm(cudaStream_t st, int n, int batch, const zc* a, long long a_stride, zc* w, zc* v, int* info, zc* ws,
                      double eps, int max_iter, int group) {
     if (batch <= 0 || n <= 0) return;
+    const bool fixed = eps == DBL_EPSILON && max_iter >= 30 && eig_fixed_enabled();
     if (group == 0) {
-        if (autotune_wanted(1, n, batch)) autotune_eig(st, 1, n, batch, a, a_stride, nullptr);
+        // A recorded form is one of the FP64 reduction. So nothing is tuned unasked where the built-in rule has the
+        // fixed-point reduction for a batch of the same key (the key's smallest).
+        int least = 1;
+        while (2LL * least <= batch) least *= 2;
+        if (!(fixed && herm_fixed_reduce_wanted(n, least)) && autotune_wanted(1, n, batch))
+            autotune_eig(st, 1, n, batch, a, a_stride, nullptr);
         group = tuned_eig_form(1, n, batch);
     }
     const size_t ysm = (size_t)n * kHermRows * sizeof(double);
@@ -301,7 +307,6 @@ void launch_eig_herm(cudaStream_t st, int n, int batch, const zc* a, long long a
     // form is forced or recorded and the batch is small (herm_fixed_reduce_wanted). Divide and conquer takes d, e and Q
     // of every matrix as they come, so it follows a reduction that writes them for every matrix: the fixed-point one
     // leaves those of a matrix that it declines (zero, not finite, far out of scale) unwritten.
-    const bool fixed = eps == DBL_EPSILON && max_iter >= 30 && eig_fixed_enabled();
     const bool dc = real_form && herm_dc_wanted(group > 0 ? group : eig_default_group(n, batch));
     const bool fixed_reduce = fixed && !dc && group == 0 && herm_fixed_reduce_wanted(n, batch);
     if (group <= 0) group = eig_default_group(n, batch);
