@@ -42,12 +42,11 @@ void fix_apply(cudaStream_t st, int n, int batch, zc* z, long long z_stride, con
         fix_apply_rows<32>(st, n, batch, z, z_stride, log, log_stride, table, head, status);
 }
 
-template <bool Herm>
 void fix_range(cudaStream_t st, int n, int batch, const zc* a, long long a_stride, int* status, int other) {
     // Small CTAs where there are many matrices: they find room beside another stream's kernels (the mirror sweep, 4096 matrices
     // of order 121 a stream, 363.8 ms without this kernel: 365.1 with 64 threads, 365.8 with 128, 366.0 with 512).
     const int threads = batch >= 608 ? 64 : kFixRangeThreads;
-    fix_range_kernel<Herm><<<(unsigned)batch, threads, fix_range_smem(n), st>>>(n, batch, a, a_stride, status, other);
+    fix_range_kernel<<<(unsigned)batch, threads, fix_range_smem(n), st>>>(n, batch, a, a_stride, status, other);
     ++launch_count();
     RCWA_CUDA(cudaGetLastError());
 }
@@ -80,8 +79,6 @@ void launch_eig_fixed(cudaStream_t st, int n, int batch, const zc* a, long long 
     const int chunk = (int)std::max(1LL, std::min<long long>(std::min(batch, std::max(kFixPassMin, (batch + 1) / 2)),
                                                              kFixLogBytes / eig_fixed_bytes(n)));
     DeviceScratch mem(st);
-    int* other = mem.get<int>(batch);
-    fix_range<false>(st, n, batch, a, a_stride, other, 1);
     int4* log = mem.get<int4>((size_t)chunk * 2 * fix_log_capacity(n));
     int4* table = mem.get<int4>((size_t)chunk * fix_table_capacity(n));
     int *head = mem.get<int>((size_t)chunk * 2), *status = mem.get<int>(chunk);
@@ -93,7 +90,7 @@ void launch_eig_fixed(cudaStream_t st, int n, int batch, const zc* a, long long 
         zc *z1 = wsc + nn, *z2 = wsc + 2 * nn;  // Z; X
         lz* h = reinterpret_cast<lz*>(wsc);
         fix_schur_kernel<false><<<(unsigned)cb, 32 * warps, schur_smem, st>>>(n, cb, ac, a_stride, wc, h, wst, log, 2 * fix_log_capacity(n), table, head, status,
-                                                                       done + b0, info + b0, other + b0);
+                                                                       done + b0, info + b0, nullptr, true);
         RCWA_CUDA(cudaGetLastError());
         fix_apply(st, n, cb, z1, wst, log, 2 * fix_log_capacity(n), table, head, status);
         zc* t = t_out ? t_out + (long long)b0 * nn : vc;
@@ -117,7 +114,7 @@ void launch_eig_fixed(cudaStream_t st, int n, int batch, const zc* a, long long 
 
 // status[b] = kFixOther for a matrix that the FP64 reduction and QL iteration keep, else 0
 void launch_herm_range(cudaStream_t st, int n, int batch, const zc* a, long long a_stride, int* status) {
-    fix_range<true>(st, n, batch, a, a_stride, status, kFixOther);
+    fix_range(st, n, batch, a, a_stride, status, kFixOther);
 }
 
 // The Hermitian solver's reduction: d and e into ws (where the QL kernel reads them) and Q (n x n, contiguous);
@@ -130,7 +127,7 @@ void launch_herm_reduce_fixed(cudaStream_t st, int n, int batch, const zc* a, lo
     DeviceScratch mem(st);
     int4* log = mem.get<int4>((size_t)batch * log_stride);
     int *head = mem.get<int>((size_t)batch * 2), *other = mem.get<int>(batch);
-    fix_range<true>(st, n, batch, a, a_stride, other, 1);
+    fix_range(st, n, batch, a, a_stride, other, 1);
     fix_schur_kernel<true><<<(unsigned)batch, 32 * warps, schur_smem, st>>>(n, batch, a, a_stride, nullptr, reinterpret_cast<lz*>(ws), wst,
                                                                             log, log_stride, nullptr, head, status, nullptr, nullptr, other);
     RCWA_CUDA(cudaGetLastError());

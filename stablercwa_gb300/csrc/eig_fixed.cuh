@@ -334,12 +334,11 @@ __device__ __forceinline__ void fix_shared_max(int* p, int v) {
 #endif
 }
 
-// status[b]: `other` for a matrix that the FP64 kernels keep, else 0. A CTA per matrix, which it reads once (a warp takes
+// Hermitian matrices; status[b]: `other` for one that the FP64 kernels keep, else 0. A CTA per matrix, which it reads once (a warp takes
 // 32 rows of eight columns at a time, all loads in flight); then a warp for every small row or column. Latency bounds it
 // for one matrix (order 121: 11 us cold; with 128 threads, 32 rows and all columns a warp, 65), the memory for 4096 (0.18 ms).
-template <bool Herm>
-__global__ void __launch_bounds__(kFixRangeThreads) fix_range_kernel(int n, int batch, const zc* __restrict__ a_in, long long a_stride,
-                                                                     int* __restrict__ status, int other) {
+static __global__ void __launch_bounds__(kFixRangeThreads) fix_range_kernel(int n, int batch, const zc* __restrict__ a_in,
+                                                                            long long a_stride, int* __restrict__ status, int other) {
     RCWA_DYN_SMEM(int, fix_rg);
     const long long gid = blockIdx.x;
     if (gid >= batch) return;
@@ -362,7 +361,7 @@ __global__ void __launch_bounds__(kFixRangeThreads) fix_range_kernel(int n, int 
         for (int u = 0; u < 8; ++u) {
             const int c = min(c0 + u, n - 1);
             m = max(m, v[u]);
-            outside |= in && v[u] != 0 && (Herm ? c + 1 < r || r + 1 < c : c < r);
+            outside |= in && v[u] != 0 && (c + 1 < r || r + 1 < c);
             const int w = fix_warp_max(in ? v[u] : 0);
             if (lane == u) col = w;
         }
@@ -373,31 +372,26 @@ __global__ void __launch_bounds__(kFixRangeThreads) fix_range_kernel(int n, int 
     __syncthreads();
     int top = 0, high = 0;  // the largest, and 2^31 - 1 less the smallest that is not zero
     for (int i = lane; i < n; i += 32) {
-        if (Herm && warp == 0) rs[i] = max(rs[i], cs[i]);
+        if (warp == 0) rs[i] = max(rs[i], cs[i]);
         const int m = max(rs[i], cs[i]);
         top = max(top, m);
         if (m) high = max(high, 0x7fffffff - m);
     }
     top = fix_warp_max(top);
     const int low = 0x7fffffff - fix_warp_max(high);
-    if (Herm) __syncthreads();
+    __syncthreads();
     bool keep = false;
-    if (top != 0 && top < 0x7ff00000) {  // zero and non-finite matrices are the solvers' own to leave
-        if (!Herm) {
-            int last = n - 1;
-            while (min(rs[last], cs[last]) == 0 && last > 0) --last;
-            keep = !flags[0] || min(rs[last], cs[last]) + kFixRangeSmall <= top;
-        } else if (low + kFixRangeSmall <= top) {
-            keep = !flags[0];
-            for (int i = warp; i < n; i += nw) {
-                const int m = rs[i];
-                if (m == 0 || m + kFixRangeSmall > top) continue;
-                const bool far = m + kFixRangeFar <= top;
-                int tie = 0;
-                for (int k = lane; k < n; k += 32)
-                    if (rs[k] >= m + (far ? kFixRangeSmall : kFixRangeLarger)) tie = max(tie, max(fix_magnitude(A[(long long)k * n + i]), fix_magnitude(A[(long long)i * n + k])));
-                keep |= fix_warp_max(tie) + (far ? kFixRangeTie : kFixRangeUntied) <= m;
-            }
+    if (top != 0 && top < 0x7ff00000 && low + kFixRangeSmall <= top) {  // zero and non-finite matrices are the solver's own to leave
+        keep = !flags[0];
+        for (int i = warp; i < n; i += nw) {
+            const int m = rs[i];
+            if (m == 0 || m + kFixRangeSmall > top) continue;
+            const bool far = m + kFixRangeFar <= top;
+            int tie = 0;
+            for (int k = lane; k < n; k += 32)
+                if (rs[k] >= m + (far ? kFixRangeSmall : kFixRangeLarger))
+                    tie = max(tie, max(fix_magnitude(A[(long long)k * n + i]), fix_magnitude(A[(long long)i * n + k])));
+            keep |= fix_warp_max(tie) + (far ? kFixRangeTie : kFixRangeUntied) <= m;
         }
     }
     if (keep) flags[1] = 1;
@@ -405,26 +399,51 @@ __global__ void __launch_bounds__(kFixRangeThreads) fix_range_kernel(int n, int 
     if (tid == 0) status[gid] = flags[1] ? other : 0;
 }
 
+// The general solver's, by all threads of its CTA (flags: 4 slots a warp), in its own kernel: as a launch of its own it took 0.9 %
+// of a sweep of small batches (two gratings, 128 samples of order 61: 25.85 to 26.07 ms), so 25.85.
+__device__ __forceinline__ bool fix_keeps_fp64(int n, const zc* __restrict__ A, int* flags) {
+    const int tid = threadIdx.x, nthr = blockDim.x, nw = nthr >> 5;
+    int v[4] = {0, 0, 0, 0};  // the largest, in the last row, in the last column, below the diagonal
+    for (int r = tid; r < n; r += nthr)
+#pragma unroll 8
+        for (int c = 0; c < n; ++c) {
+            const int m = fix_magnitude(A[(long long)c * n + r]);
+            v[0] = max(v[0], m);
+            if (r == n - 1) v[1] = max(v[1], m);
+            if (c == n - 1) v[2] = max(v[2], m);
+            if (r > c) v[3] = max(v[3], m);
+        }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int m = fix_warp_max(v[q]);
+        if ((tid & 31) == 0) flags[4 * (tid >> 5) + q] = m;
+    }
+    __syncthreads();
+    for (int w = 0; w < nw; ++w)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) v[q] = max(v[q], flags[4 * w + q]);
+    __syncthreads();
+    return v[3] == 0 || min(v[1], v[2]) + kFixRangeSmall <= v[0];
+}
+
 constexpr int kFixBatch = 6;  // columns whose entries a row's lane holds at once, and as many on their way
 
 // Schur reduction of one matrix; with Herm only step 1, on the Hermitian part (A + A^H) / 2: the reduced matrix is
 // real symmetric tridiagonal, its d and e go where the QL kernel reads them. H: n x n lz (column-major, global). log: rotations (two int4 each), table:
 // (l, en, phase) per sweep in int4. w: eigenvalues in deflation order. status: 0 done, 1 left to the FP64
-// kernels (non-finite input, no convergence, log full). head: the
+// kernels (non-finite input, no convergence, log full; other[b] set, or `check` and fix_keeps_fp64). head: the
 // number of sweeps and the exponent of the unit.
 template <bool Herm>
 __global__ void fix_schur_kernel(int n, int batch, const zc* __restrict__ a_in, long long a_stride, zc* __restrict__ w_out,
                                         lz* __restrict__ h_ws, long long h_stride, int4* __restrict__ log_all, long long log_stride,
                                         int4* __restrict__ table_all, int* __restrict__ head, int* __restrict__ status,
-                                        int* __restrict__ done, int* __restrict__ info, const int* __restrict__ other = nullptr) {
+                                        int* __restrict__ done, int* __restrict__ info, const int* __restrict__ other = nullptr,
+                                        bool check = false) {
     RCWA_DYN_SMEM(lz, fix_sm);
     const long long gid = blockIdx.x;
     if (gid >= batch) return;
     if (other && other[gid]) {
-        if (threadIdx.x == 0) {
-            status[gid] = 1;
-            if (!Herm) done[gid] = 0;
-        }
+        if (threadIdx.x == 0) status[gid] = 1;
         return;
     }
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nthr = blockDim.x, nw = nthr >> 5;
@@ -442,6 +461,15 @@ __global__ void fix_schur_kernel(int n, int batch, const zc* __restrict__ a_in, 
     const long long nn = (long long)n * n;
     const lz zero{0, 0};
 
+    if constexpr (!Herm) {
+        if (check && fix_keeps_fp64(n, A, flags)) {
+            if (tid == 0) {
+                status[gid] = 1;
+                done[gid] = 0;
+            }
+            return;
+        }
+    }
     // ---- scale: the largest exponent, then N (sums in a fixed order)
     int top = 0;
     for (long long i = tid; i < nn; i += nthr) {

@@ -1,4 +1,4 @@
-// Runs fix_range_kernel (stablercwa_gb300/csrc/eig_fixed.cuh) on the CPU: which matrices the fixed-point eigensolvers leave to
+// Runs fix_range_kernel and fix_keeps_fp64 (stablercwa_gb300/csrc/eig_fixed.cuh) on the CPU: which matrices the fixed-point eigensolvers leave to
 // the FP64 kernels, whose small eigenvalues those keep relative to themselves, and which they take (layer matrices of every
 // declared kind among them).
 #include <random>
@@ -16,7 +16,12 @@ static void check(const char* name, int n, const M& a, bool other) {
     for (bool descending : {false, true}) {
         if (descending && n > 2) break;
         int status = -1;
-        run_cta(kFixRangeThreads, fix_range_smem(n), [&] { fix_range_kernel<Herm>(n, 1, a.data(), (long long)n * n, &status, 2); }, descending);
+        int flags[48] = {};
+        if (Herm) run_cta(kFixRangeThreads, fix_range_smem(n), [&] { fix_range_kernel(n, 1, a.data(), (long long)n * n, &status, 2); }, descending);
+        else run_cta(128, 0, [&] {
+            const bool keep = fix_keeps_fp64(n, a.data(), flags);
+            if (threadIdx.x == 77) status = keep ? 2 : 0;
+        }, descending);
         const bool ok = status == (other ? 2 : 0);
         std::printf("%s %-36s n=%3d %s: %s\n", ok ? "pass" : "FAIL", name, n, Herm ? "Hermitian" : "general", status ? "FP64" : "fixed point");
         failures += !ok;
@@ -117,7 +122,7 @@ int main() {
         check<true>("tridiagonal, upwards", n, t, true);
         M bad = g;
         bad[n + 3] = zc{INFINITY, 0};
-        check<false>("not finite", n, bad, false);
+        check<true>("not finite", n, bad, false);
     }
     for (int n : {25, 41, 121})
         for (double step : {0.1, 1.83, 10.0})

@@ -1,4 +1,4 @@
-"""Which matrices the fixed-point eigensolvers leave to the FP64 kernels (fix_range_kernel in
+"""Which matrices the fixed-point eigensolvers leave to the FP64 kernels (fix_range_kernel, fix_keeps_fp64 in
 stablercwa_gb300/csrc/eig_fixed.cuh), compiled for the host and run through the warp-level emulation of tests/emu/warp/:
 matrices whose small eigenvalues FP64 keeps relative to themselves stay there, layer matrices do not."""
 import os
