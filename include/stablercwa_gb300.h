@@ -391,7 +391,8 @@ int rcwa_gpu_kernel_busy(rcwa_gpu_ctx* ctx, const char* kind, double* millisecon
  * max_iter >= 30 and no form forced, orders 24 to 440 are solved in 64-bit fixed point: residuals as in FP64 or smaller, every
  * eigenvalue to about 2^-58 of ||A||_2, however small it is itself. Matrices whose small eigenvalues FP64 would keep
  * relative to themselves go to the FP64 kernels: upper triangular ones, and those whose last row or column is below 2^-7
- * of the largest (graded downwards, or with a separate small block last). */
+ * of the largest (graded downwards, or with a separate small block last); last rows without entries left of the diagonal
+ * are passed over, unless a diagonal entry of one is that small. */
 int rcwa_gpu_eig_batch(rcwa_gpu_ctx* ctx, int n, int batch, const rcwa_complex* a, double eps, int max_iter,
                        rcwa_complex* values, rcwa_complex* vectors, int* info, int* sweeps);
 int rcwa_gpu_eig_batch_dev(rcwa_gpu_ctx* ctx, int n, int batch, const rcwa_complex* d_a, double eps,

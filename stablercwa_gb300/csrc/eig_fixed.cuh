@@ -292,9 +292,11 @@ __device__ __forceinline__ lz fix_left_block(int n, lz* H, lz* tile, const int4*
 // m is. FP64 loses more where its reflectors or shifts mix such a row with those of size N, as on a layer matrix
 // Kx^2 - [[eps]], whose centre is 2^-16 of N and tied to the rest by the profile's harmonics; where they do not it keeps
 // 2^-53 of the row, and such matrices stay with the FP64 kernels:
-//   - general solver: upper triangular matrices, and those whose last row or column is 2^-7 below the largest (graded
-//     downwards, or a small block last: deflated before a large shift has passed over them). A layer's last order is one
-//     of its largest (2^-4 of it at grazing incidence on a wide period).
+//   - general solver: matrices whose last row or column is 2^-7 below the largest (graded downwards, or a small block last:
+//     deflated before a large shift has passed over them). Last rows without entries left of the diagonal deflate before
+//     there is a shift: a small diagonal entry in one of them counts, and past them the last row or column of the block
+//     that is left; upper triangular matrices are nothing else. A layer's last order is one of its largest (2^-4 of it at
+//     grazing incidence on a wide period), with entries to its left.
 //   - Hermitian solver: rows 2^-7 below the largest that nothing ties to larger ones (diagonal matrices, separate blocks),
 //     in which the entries towards rows 2^3 larger are below 2^-40 of the row, or, 2^-14 below the largest, those
 //     towards rows 2^7 larger below 2^-16; and tridiagonal matrices with a row 2^-7 below the largest. The centre rows of layers,
@@ -403,7 +405,19 @@ static __global__ void __launch_bounds__(kFixRangeThreads) fix_range_kernel(int 
 // of a sweep of small batches (two gratings, 128 samples of order 61: 25.85 to 26.07 ms), so 25.85.
 __device__ __forceinline__ bool fix_keeps_fp64(int n, const zc* __restrict__ A, int* flags) {
     const int tid = threadIdx.x, nthr = blockDim.x, nw = nthr >> 5;
-    int v[4] = {0, 0, 0, 0};  // the largest, in the last row, in the last column, below the diagonal
+    int v[4] = {0, 0, 0, 0};  // the largest, in the last row, in the last column; the rows up to the last with an entry left of its diagonal
+    const auto all = [&] {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int m = fix_warp_max(v[q]);
+            if ((tid & 31) == 0) flags[4 * (tid >> 5) + q] = m;
+        }
+        __syncthreads();
+        for (int w = 0; w < nw; ++w)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) v[q] = max(v[q], flags[4 * w + q]);
+        __syncthreads();
+    };
     for (int r = tid; r < n; r += nthr)
 #pragma unroll 8
         for (int c = 0; c < n; ++c) {
@@ -411,19 +425,26 @@ __device__ __forceinline__ bool fix_keeps_fp64(int n, const zc* __restrict__ A, 
             v[0] = max(v[0], m);
             if (r == n - 1) v[1] = max(v[1], m);
             if (c == n - 1) v[2] = max(v[2], m);
-            if (r > c) v[3] = max(v[3], m);
+            if (r > c && m) v[3] = r + 1;
         }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const int m = fix_warp_max(v[q]);
-        if ((tid & 31) == 0) flags[4 * (tid >> 5) + q] = m;
+    all();
+    const int p = v[3], small = v[0] - kFixRangeSmall;
+    if (p == 0) return true;
+    if (p < n) {
+        // the rows from p on deflate before there is a shift: their diagonal entries, then the block before them
+        v[1] = v[2] = v[3] = 0;
+        for (int i = tid; i < n; i += nthr) {
+            if (i < p) {
+                v[1] = max(v[1], fix_magnitude(A[(long long)i * n + p - 1]));
+                v[2] = max(v[2], fix_magnitude(A[(long long)(p - 1) * n + i]));
+            } else if (fix_magnitude(A[(long long)i * (n + 1)]) <= small) {
+                v[3] = 1;
+            }
+        }
+        all();
+        if (v[3]) return true;
     }
-    __syncthreads();
-    for (int w = 0; w < nw; ++w)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) v[q] = max(v[q], flags[4 * w + q]);
-    __syncthreads();
-    return v[3] == 0 || min(v[1], v[2]) + kFixRangeSmall <= v[0];
+    return min(v[1], v[2]) <= small;
 }
 
 constexpr int kFixBatch = 6;  // columns whose entries a row's lane holds at once, and as many on their way

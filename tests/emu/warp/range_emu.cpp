@@ -101,6 +101,27 @@ int main() {
             for (int i = j + 1; i < n; ++i) u[(size_t)j * n + i] = zc{0, 0};
         check<false>("upper triangular", n, u, true);
         if (n < 24) continue;
+        for (int lead : {2, n / 2, n - 1}) {  // rows `lead` on without entries left of the diagonal: deflated before any shift
+            M st = u;
+            for (int j = 0; j < lead; ++j)
+                for (int i = 0; i < lead; ++i) st[(size_t)j * n + i] = g[(size_t)j * n + i];
+            for (int i = 0; i < n; ++i) st[(size_t)i * n + i] = zc{1.0 + i, 0};
+            check<false>("dense block, triangular rest", n, st, false);
+            M one_small = st;
+            one_small[(size_t)(n - 1 - (lead < n - 1)) * (n + 1)] = zc{1e-10, 0};
+            check<false>("the same, a small diagonal entry", n, one_small, true);
+            for (double small : {1e-20, 1e-5}) {
+                M sm = st, sd = st;
+                for (int j = 0; j < n; ++j)
+                    for (int i = 0; i < n; ++i) {
+                        const bool in = i < lead && j < lead;
+                        sm[(size_t)j * n + i] = st[(size_t)j * n + i] * (in ? small : 1.0);
+                        sd[(size_t)j * n + i] = st[(size_t)j * n + i] * (in ? small : i == j ? 1.0 : 0.0);
+                    }
+                check<false>("a small block first, triangular rest", n, sm, true);
+                check<false>("a small block first, diagonal rest", n, sd, true);
+            }
+        }
         for (bool first : {false, true})  // two blocks of very different size, the small one first or last
             for (double small : {1e-20, 1e-5}) {
                 M hb = h, gb = g;
