@@ -228,7 +228,8 @@ typedef struct rcwa_result2d {
 
 typedef struct rcwa_gpu_config {
     int device;                /* CUDA device ordinal */
-    size_t workspace_limit;    /* bytes of device workspace the context may hold; 0 = 8 GiB */
+    size_t workspace_limit;    /* bytes of device workspace a call may hold; 0 = half the free memory, at most 48 GiB (crossed
+                                  gratings 80 % of what is free or cached); a single point is solved whatever it takes */
 } rcwa_gpu_config;
 
 typedef struct rcwa_gpu_ctx rcwa_gpu_ctx;

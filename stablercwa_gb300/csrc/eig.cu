@@ -264,7 +264,8 @@ bool herm_blocked_wanted(int n, int group) {
 // from order 64, there with fixed-point panels), whole eigensolves in ms: order 41: 1 matrix 2.0 / 2.7, 4000 12.5 / 10.5;
 // order 61: 1 4.2 / 5.8, 1000 10.1 / 11.0; order 81: 304 9.8 / 10.6, 592 14.1 / 12.7; order 121: 64 17.2 / 23.2, 304
 // 23.4 / 25.0, 396 30.1 / 27.6; order 161: 298 54 / 68; order 301: 16 115 / 213, 159 275 / 308. The line lies where
-// n * batch matrices' columns fill the GPU's SMs about three deep, for the blocked form at most 360 matrices.
+// n * batch matrices' columns fill the GPU's SMs about three deep, for the blocked form at most 360 matrices. From order
+// 161 on the fixed-point form still wins on the line; where the forms meet beyond it has not been measured.
 bool herm_fixed_reduce_wanted(int n, int batch) {
     return (long long)n * batch <= 48000 && (n < 64 || batch <= 360) && eig_fixed_possible(n);
 }

@@ -11,9 +11,10 @@ namespace {
 // largest order: 32 rows of Z (16 bytes an entry) and the back substitution's slots in 227 KB of shared memory
 constexpr int kFixMaxOrder = 440;
 constexpr int kFixMinOrder = 24;
-// Matrices per pass: the logs (about 96 n^2 bytes each) of half the batch, so that they stay within what the
-// callers' estimates leave beside the eigensolver's workspace, but of three matrices an SM at least and of 4 GB
-// at most.
+// Matrices per pass: the logs (about 96 n^2 bytes each) of half the batch, but of three matrices an SM at least and of
+// 4 GB at most. The 2-D solver counts them in its estimate of a point; in the 1-D and conical ones they are freed before
+// the dense operators that the estimate is made for come to be: calls with a limit of 1024 MiB held at most 942 (1-D,
+// orders 31 to 301) and 987 MiB (conical, 25 to 121), absorbing or not, with one grating or three.
 constexpr int kFixPassMin = 456;
 constexpr long long kFixLogBytes = 4LL << 30;
 

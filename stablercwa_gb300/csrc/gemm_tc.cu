@@ -21,7 +21,7 @@
 // Kernels. The split kernels write the digit planes in HBM as bf16 rows with K contiguous (K-major for
 // both operands), the second half of a complex K starting at Kp / 2. The product kernel gives each CTA one
 // 128 x 128 tile of C^ of one matrix: one warp issues TMA loads (128-byte swizzle, boxes of 128 rows x 64 K, two
-// of each operand a stage) into a 3-stage shared-memory ring; one thread issues tcgen05.mma (M = 128, N = 256 or 128,
+// of each operand a stage: two digits of 64 K, or one of 128 K) into a 3-stage shared-memory ring; one thread issues tcgen05.mma (M = 128, N = 256 or 128,
 // K = 16, bf16 in, FP32 out) into four 128-column tensor-memory accumulators; eight warps read each finished
 // accumulator out of tensor memory (tcgen05.ld) and add it, as an integer at its diagonal's weight, into one int64 per
 // element while the next group accumulates in other slots, then convert once, apply 2^(ea + eb), pair the
@@ -50,9 +50,10 @@
 namespace rcwa_gb300 {
 namespace {
 
-// A stage holds 128 K of both operands (64 bf16 = one 128-byte swizzle row a box): with the 64 K of an earlier form
-// the issuing thread's wait, eight descriptors and commit took 560 cycles a stage against the 256 of its four
-// MMAs; eight MMAs a stage and descriptors that are additions keep the tensor pipe ahead.
+// A stage holds two boxes of each operand (64 bf16 = one 128-byte swizzle row a box): of a quad 64 K of two digits of
+// each, in eight MMAs (nine where an accumulator's first product has to be issued on its own), of a pair 128 K of one
+// digit of each, in eight. With one box each the issuing thread's wait, descriptors and commit took 560 cycles a stage
+// against the 256 of its four MMAs; eight MMAs a stage and descriptors that are additions keep the tensor pipe ahead.
 constexpr int kTileM = 128, kTileN = 128, kTileK = 64;
 constexpr int kStageBoxes = 2;
 constexpr int kStages = 3;

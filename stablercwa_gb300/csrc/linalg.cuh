@@ -523,12 +523,12 @@ __global__ void lu_nan_fill_kernel(int n, int nrhs, int batch, zc* x, long long 
     if (idx - sys * per == 0) singular[sys] = 1;
 }
 
-// Batched complex GEMM: C = s_ab * (A B) + s_c * C0, one warp per 32 x COLS tile of C, lanes along rows (COLS 8, or 2
-// where 8 would leave schedulers without a warp: a step over k is 4 COLS FP64 instructions of 64 cycles).
+// Batched complex GEMM: C = s_ab * (A B) + s_c * C0, one warp per 32 x COLS tile of C, lanes along rows (COLS 8, or 2 or
+// 1 where more would leave schedulers without a warp: a step over k is 4 COLS FP64 instructions of 64 cycles).
 // A: m x k (lda), B: k x n (ldb), C/C0: m x n (ldc); any stride may be 0 to broadcast one operand
 // to the whole batch. s_ab, s_c in {-1, 0, 1}. C may alias C0 (each element is read then written by
-// the same lane). The sum over k runs in ascending order, as the reference's column GEMM adds
-// (include/stablercwa/matrix.hpp:170-192).
+// the same lane). The sums over k run in ascending order, as the reference's column GEMM adds
+// (include/stablercwa/matrix.hpp:170-192); with COLS 1 and 2 the two products of each part have a sum of their own.
 template <int COLS>
 __global__ void __launch_bounds__(128) zgemm_kernel(int m, int n, int k, int batch, const zc* __restrict__ A, int lda,
                                                     long long a_stride, const zc* __restrict__ B, int ldb,

@@ -53,10 +53,9 @@ __global__ void col_extract_kernel(int B, int n, const zc* __restrict__ m, int c
     out[((long long)b * ocols + oc) * n + i] = m[(long long)b * n * n + (long long)col * n + i];
 }
 
-// y = s_c * y0 + s_ab * (A x), warp per sample, lanes along rows; the sum over columns is ascending
-// like the reference's matrix-vector product (include/stablercwa/matrix.hpp:186-194).
-// A CTA per sample and 32 rows: a lane per row, the columns of A dealt to its four warps, their sums added in order
-// through shared memory. (A warp per sample took 1.0 ms for one matrix of order 338 on one SM.)
+// y = s_c * y0 + s_ab * (A x) (include/stablercwa/matrix.hpp:186-194). A CTA per sample and 32 rows: a lane per row; its
+// four warps take every fourth column each, and their sums are added as (0 + 1) + (2 + 3) through shared memory: four
+// shorter ascending sums in place of one. (A warp per sample took 1.0 ms for one matrix of order 338 on one SM.)
 constexpr int kMatvecThreads = 128;
 inline dim3 matvec_grid(int B, int n) { return dim3((unsigned)B, (unsigned)((n + 31) / 32)); }
 __device__ __forceinline__ zc matvec_row(int n, int i, const zc* __restrict__ As, const zc* __restrict__ xs) {
