@@ -12,9 +12,10 @@ value      solves/s with inputs resident in device memory (the *_dev C entry poi
            polarizations per call), timed with CUDA events on the engine's stream, L2 flushed between steps.
 e2e        the same metric through the host-buffer C entry point (host -> device copy of the points
            and device -> host copy of all results inside the timed region).
-roofline   the eigensolve stage (the dominant stage; for the grating's real permittivities its three
-           Hermitian kernels): algorithmic FP64 flops per launch / its event-timed duration, against the
-           FP64 peak measured here with cuBLAS DGEMM.
+roofline   the eigensolve stage (the dominant stage): its algorithmic FP64 flops per launch / its event-timed
+           duration, beside the FP64 peak measured here with cuBLAS DGEMM. The stage runs in fixed point on the
+           integer pipes and in digits on the tensor cores, so their ratio (ratio_to_dgemm) is no fraction of what
+           bounds it; frac is given where the FP64 kernels run. hbm: its DRAM bytes against the measured copy rate.
 cpu_baseline  the CPU oracle (a C++ restatement of the reference's solve) on the host cores.
 --impl reference  times that CPU implementation alone on the same workload definition.
 """
@@ -59,16 +60,40 @@ def workload(seed=SEED, n_points=N_POINTS, ridge=1.46):
     return stack, pts, {"fill": float(fill), "depth": float(depth)}
 
 
-# DRAM bytes per matrix of the Hermitian eigensolve stage at n = 121 (blocked tridiagonalisation 22.0 MB,
-# its tensor-core trailing updates and the back-transformation with their digit splits 8.5 MB, QL 0.3 MB,
-# rotations on the real identity 1.2 MB, the rest 1.0 MB), from one ncu capture of every launch of one
-# 4096-matrix eigensolve of this order
-HERM_STAGE_DRAM_BYTES_PER_MATRIX_N121 = 33.0e6
+# DRAM bytes per matrix of the Hermitian eigensolve stage at n = 121 (fixed-point panels of the tridiagonalisation
+# 18.1 MB, its tensor-core trailing updates and the back-transformation with their digit splits 9.0 MB, rotations on
+# the real identity 1.2 MB, QL 0.2 MB, the rest 0.7 MB), from one ncu capture of every launch of one 1024-matrix
+# eigensolve of this order
+HERM_STAGE_DRAM_BYTES_PER_MATRIX_N121 = 29.2e6
 
 
 HERM_STAGE_KERNELS = ("eigensolve stage: herm_panel_fixed_kernel (blocked tridiagonalisation, fixed point) + tensor-core "
                       "trailing updates + herm_ql_fixed_kernel + herm_apply_real_kernel (QL and its rotations on a real "
                       "identity in 64-bit fixed point on the integer pipes) + tensor-core back-transformation")
+
+
+def general_eig_kernel(n):
+    """The kernel that carries the general eigensolver at order n, and whether it is a fixed-point one."""
+    fixed = 24 <= n <= 440 and not os.environ.get("RCWA_GB300_EIG_FIXED", "").startswith("0")
+    return ("fix_schur_kernel", True) if fixed else ("eig_block_kernel (eig_cluster_kernel for up to 64 matrices)", False)
+
+
+def eig_rate(achieved, peak, flops_model, fixed):
+    """The eigensolve stage's rate in algorithmic FP64 operations beside cuBLAS DGEMM's. Only the FP64 kernels are bound by
+    the pipe that DGEMM runs on; the fixed-point ones wait for their own chains, with no integer pipe above 37 %."""
+    ratio = achieved / peak if achieved else None
+    return {"bound": "latency (fixed-point kernels, few warps an SM)" if fixed else "fp64", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
+            "frac": None if fixed else ratio, "ratio_to_dgemm": ratio, "flops_model": flops_model,
+            "peak_source": "measured in this run: cuBLAS DGEMM 4096^3 (torch.matmul float64), best of 5"}
+
+
+def copy_rate_gbs():
+    """The measured HBM copy rate of this GPU, if it was recorded."""
+    path = os.path.join(ROOT, "MEASURED_PEAKS.json")
+    if not os.path.exists(path):
+        return None
+    with open(path) as f:
+        return json.load(f).get("hbm_gbs")
 
 
 def herm_flops_text(n, rotations_per_matrix):
@@ -387,6 +412,10 @@ def run_ours(args):
     # one was running (union of their CUDA-event intervals on the two streams)
     achieved = eig_flops_launch * eig_launches / (eig_busy_ms * 1e-3) / 1e12
     step_ms = total_ms / args.steps
+    fixed = general_eig_kernel(n)[1]
+    traffic = HERM_STAGE_DRAM_BYTES_PER_MATRIX_N121 * P if herm and n == 121 and fixed else None
+    hbm_gbs = traffic * eig_launches / (eig_busy_ms * 1e-3) / 1e9 if traffic else None
+    copy_gbs = copy_rate_gbs()
     if rank == 0:
         line = {"metric": METRIC, "value": value, "unit": "solves/s", "n_gpus": world, "steps": args.steps,
                 "warmup": args.warmup, "ms_per_step": step_ms, "higher_is_better": True, "scaling": "weak",
@@ -398,17 +427,15 @@ def run_ours(args):
                 "clocks": clocks,
                 "e2e": {"value": e2e_value, "unit": "solves/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h},
                 "gpu_launches": launches,
-                "roofline": {"bound": "fp64", "kernel": (HERM_STAGE_KERNELS if herm else "fix_schur_kernel"),
-                             "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
-                             "traffic": (HERM_STAGE_DRAM_BYTES_PER_MATRIX_N121 * P
-                                         if herm and n == 121 and HERM_STAGE_DRAM_BYTES_PER_MATRIX_N121 else None),
+                "roofline": {"kernel": HERM_STAGE_KERNELS if herm else general_eig_kernel(n)[0],
+                             **eig_rate(achieved, peak, herm_flops_text(n, rot_per_matrix) if herm
+                                        else "general QR: 105 n^3 per matrix", fixed),
+                             "traffic": traffic,
                              "traffic_source": ("ncu dram__bytes_read.sum + dram__bytes_write.sum of every launch of "
-                                                "one eigensolve call per matrix (4096-matrix capture) x matrices per "
-                                                "launch" if herm and n == 121 and HERM_STAGE_DRAM_BYTES_PER_MATRIX_N121
-                                                else None),
-                             "flops_model": (herm_flops_text(n, rot_per_matrix) if herm
-                                             else "general QR: 105 n^3 per matrix"),
-                             "peak_source": "measured in this run: cuBLAS DGEMM 4096^3 (torch.matmul float64), best of 5",
+                                                "one eigensolve call per matrix (1024-matrix capture) x matrices per "
+                                                "launch" if traffic else None),
+                             "hbm": {"achieved": hbm_gbs, "peak": copy_gbs, "unit": "GB/s",
+                                     "frac": hbm_gbs / copy_gbs if hbm_gbs and copy_gbs else None},
                              "flops_per_launch": eig_flops_launch, "avg_launch_ms": eig_avg_ms,
                              "launches": eig_launches, "busy_ms": eig_busy_ms,
                              "timing": "TE and TM eigensolves run concurrently on two streams; achieved = "
@@ -500,8 +527,7 @@ def lossy_rate(eng, torch, est, flush, args, peak):
             "gpu_launches": launches, "ridge_index": [LOSSY_RIDGE.real, LOSSY_RIDGE.imag],
             "eigensolver": "general: Hessenberg reduction + shifted complex QR + back substitution (fix_schur_kernel, 64-bit fixed point)",
             "eig_ms_per_step": eig_ms, "eig_busy_ms_per_step": eig_busy,
-            "eig_roofline": {"achieved": achieved, "peak": peak, "unit": "TFLOP/s",
-                             "frac": achieved / peak if achieved else None, "flops_model": "105 n^3 per matrix"},
+            "eig_roofline": eig_rate(achieved, peak, "105 n^3 per matrix", general_eig_kernel(n)[1]),
             "accuracy": {"max_abs_dDE_vs_oracle": err, "sample_solves": 2 * len(idx),
                          "all_status_ok": bool((host["status"] == 0).all())}}
 
@@ -632,7 +658,9 @@ def run_secondary(args):
     # launch cost a little)
     eng.set_kernel_timing(True)
     step()
-    roof_kernel, flops_model = "fix_schur_kernel", "general QR: 105 n^3 per matrix"
+    flops_model = "general QR: 105 n^3 per matrix"
+    roof_kernel, fixed = general_eig_kernel(2 * (2 * CROSSED_M + 1) ** 2 if args.workload == "crossed2d" else
+                                            2 * (CONICAL_M if args.workload == "conical" else M) + 1)
     if herm_model and not os.environ.get("RCWA_GB300_HERMITIAN", "").startswith("0"):
         # lossless layers: the Hermitian eigensolver; the model counts its matrices only (the few conical
         # Schur-basis eigensolves of order 2N inside the same timer are not counted)
@@ -653,9 +681,7 @@ def run_secondary(args):
             "vs_baseline": None, "dtype": "f64 (complex128)", "data": "synthetic (seeded)", "config": config,
             "clocks": clocks, "e2e": {"value": value, "unit": "solves/s", "note": "host-buffer entry point"},
             "gpu_launches": launches,
-            "roofline": {"bound": "fp64", "kernel": roof_kernel, "achieved": achieved, "peak": peak,
-                         "unit": "TFLOP/s", "frac": achieved / peak if achieved else None, "flops_model": flops_model,
-                         "peak_source": "measured in this run: cuBLAS DGEMM 4096^3 (torch.matmul float64), best of 5"},
+            "roofline": {"kernel": roof_kernel, **eig_rate(achieved, peak, flops_model, fixed)},
             "kernels_ms_per_step": {"eig": eig_ms, "lu": lu_ms, "gemm": gemm_ms,
                                     "other": 1e3 * step_s - (eig_ms + lu_ms + gemm_ms),
                                     "note": "one instrumented step run after the timed ones"}}
