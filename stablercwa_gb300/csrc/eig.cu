@@ -29,6 +29,20 @@ int eig_default_group(int n, int batch) {
 }
 
 namespace {
+// Launches a fixed-point form; false where the device has no memory left for what that needs besides the FP64 form's
+// workspace (the rotation logs, about 96 n^2 bytes a matrix, up to 4 GB): the FP64 form takes the whole call then.
+template <class F>
+bool launched_in_memory(F&& launch) {
+    try {
+        launch();
+    } catch (const EngineError& e) {
+        if (e.code != RCWA_ENOMEM) throw;
+        cudaGetLastError();  // the failed allocation is not the next launch's error
+        return false;
+    }
+    return true;
+}
+
 // the FP64 kernels with `group` lanes or threads per matrix
 void launch_eig_fp64(cudaStream_t st, int n, int batch, const zc* a, long long a_stride, zc* w, zc* v, int* info, int* sweeps,
                      zc* ws, double eps, int max_iter, int group, const int* skip, int skip_value, zc* t_out);
@@ -44,7 +58,7 @@ void launch_eig(cudaStream_t st, int n, int batch, const zc* a, long long a_stri
         TimedLaunch timed(TK_EIG, st);
         DeviceScratch mem(st);
         int* done = mem.get<int>(batch);
-        launch_eig_fixed(st, n, batch, a, a_stride, w, v, info, ws, done, eps, t_out);
+        if (!launched_in_memory([&] { launch_eig_fixed(st, n, batch, a, a_stride, w, v, info, ws, done, eps, t_out); })) done = nullptr;
         launch_eig_fp64(st, n, batch, a, a_stride, w, v, info, sweeps, ws, eps, max_iter, eig_default_group(n, batch), done, 1,
                         t_out);
         return;
@@ -309,7 +323,7 @@ void launch_eig_herm(cudaStream_t st, int n, int batch, const zc* a, long long a
     // of every matrix as they come, so it follows a reduction that writes them for every matrix: the fixed-point one
     // leaves those of a matrix that it declines (zero, not finite, far out of scale) unwritten.
     const bool dc = real_form && herm_dc_wanted(group > 0 ? group : eig_default_group(n, batch));
-    const bool fixed_reduce = fixed && !dc && group == 0 && herm_fixed_reduce_wanted(n, batch);
+    bool fixed_reduce = fixed && !dc && group == 0 && herm_fixed_reduce_wanted(n, batch);
     if (group <= 0) group = eig_default_group(n, batch);
     TimedLaunch timed(TK_EIG, st);
     DeviceScratch mem(st);
@@ -334,10 +348,12 @@ void launch_eig_herm(cudaStream_t st, int n, int batch, const zc* a, long long a
         mall = mem.get<zc>((size_t)batch * pnb * n);
         u = mem.get<zc>((size_t)batch * kHermNb * n);
         herm_blocked_reduce(st, n, batch, a, a_stride, ws, pan, q, mall, group, fixed, status);
-    } else if (fixed_reduce) {
-        launch_herm_reduce_fixed(st, n, batch, a, a_stride, q, ws, status);
     } else {
-        herm_reduce_dispatch(st, n, batch, a, a_stride, q, ws, group);
+        if (fixed_reduce && !launched_in_memory([&] { launch_herm_reduce_fixed(st, n, batch, a, a_stride, q, ws, status); })) {
+            fixed_reduce = false;
+            launch_herm_range(st, n, batch, a, a_stride, status);
+        }
+        if (!fixed_reduce) herm_reduce_dispatch(st, n, batch, a, a_stride, q, ws, group);
     }
     const size_t qsm = (size_t)2 * n * kHermQlThreads * sizeof(double);
     if (dc) {

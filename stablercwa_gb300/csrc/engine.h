@@ -105,7 +105,8 @@ void launch_eig_cluster(cudaStream_t st, int n, int batch, const zc* a, long lon
                         int* sweeps, zc* ws, double eps, int max_iter, const int* skip, int skip_value, zc* t_out);
 // The general eigensolver with its unitary transformations in fixed point (eig_fixed.cu), for orders it can hold
 // (eig_fixed_possible): done[b] = 1 for every matrix it finished (info[b] = 0), 0 for one it leaves to the FP64
-// kernels. ws as launch_eig's; it allocates eig_fixed_bytes(n) a matrix besides (up to 4 GB at a time).
+// kernels. ws as launch_eig's; it allocates eig_fixed_bytes(n) a matrix besides (up to 4 GB at a
+// time); where the device has not got that, launch_eig takes the FP64 kernels.
 bool eig_fixed_possible(int n);
 long long eig_fixed_bytes(int n);
 void launch_eig_fixed(cudaStream_t st, int n, int batch, const zc* a, long long a_stride, zc* w, zc* v, int* info, zc* ws,
